@@ -43,6 +43,9 @@
 //                      and a row of 8 codes per row, no rowptr
 //   cg_a_ellv_kernel   other pattern matrices: a pattern byte and a row of 6
 //                      or 8 values (doubles, or floats when exact) per row
+//
+// A pattern matrix whose vectors fit the SMs is solved by cg_resident.cu
+// instead, in one launch with the vectors on the chip.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -51,6 +54,7 @@
 #include "gb_internal.h"
 #include "spmv_tiles.cuh"
 #include "cg_common.cuh"
+#include "cg_resident.h"
 
 namespace gb {
 
@@ -1055,6 +1059,12 @@ struct gb_cg {
   void * ellv = nullptr;   // [n * width] values per row (cg_a_ellv_kernel)
   bool ellv_f32 = false;   // ellv holds floats (every value exactly a float)
   gb::MixedCg * mixed = nullptr;  // GB_CG_MIXED solver (owns its workspace)
+  gb::ResidentCg * resident = nullptr;  // the solve on the chip, when the system fits
+  // GB_CG_MIXED on the chip: the solution over the refinements, and b - A x
+  double * xsum = nullptr;
+  unsigned * ticket = nullptr;
+  double * rr_true_h = nullptr;  // pinned, mapped
+  double * rr_true_d = nullptr;
 };
 
 namespace gb {
@@ -1064,6 +1074,7 @@ void destroy_cg(gb_cg * s) {
   if (!s) return;
   cudaDeviceSynchronize();  // its memory goes back to the pool below
   mixed_destroy(s->mixed);
+  resident_destroy(s->resident);
   free_row_codec(s->codec);
   free_row_patterns(s->pat);
   dev_free(s->ell8);
@@ -1080,6 +1091,9 @@ void destroy_cg(gb_cg * s) {
   dev_free(s->partial_b);
   dev_free(s->longdot);
   dev_free(s->st);
+  dev_free(s->xsum);
+  dev_free(s->ticket);
+  pinned_slot_free(s->rr_true_h);
   dev_free(s->cta_tiles);
   dev_free(s->sync);
   pinned_slot_free(s->host_status);
@@ -1201,6 +1215,71 @@ int capture_chunk(gb_cg * s, int slot) {
   return GOOSEBERRY_SUCCESS;
 }
 
+// A pattern matrix's values (or their codes) in rows of 6 or 8, which need no
+// rowptr; nothing for other matrices.  The codec is built.
+int build_ell(const gb_csr * a, gb_cg * s) {
+  if (s->codec.stage != 5 && s->codec.stage != 7) return GOOSEBERRY_SUCCESS;
+  GB_TRY(build_row_patterns(*a, &s->pat, nullptr));
+  if (s->pat.code8) {
+    const size_t rows = std::max<size_t>(s->n, 1);
+    const unsigned g = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(
+        (s->n + 255) / 256, static_cast<size_t>(a->sm_count) * 8)));
+    const uint32_t nr = static_cast<uint32_t>(s->n);
+    if (s->codec.code8) {
+      GB_TRY(dev_alloc(&s->ell8, rows * sizeof(uint2)));
+      ell8_codes_kernel<<<g, 256>>>(nr, a->rowptr, s->codec.code8, s->ell8);
+    } else if (s->codec.val32) {
+      GB_TRY(dev_alloc(&s->ellv, rows * 8 * sizeof(float)));
+      ell_vals_kernel<float, 8><<<g, 256>>>(nr, a->rowptr, s->codec.val32,
+          static_cast<float *>(s->ellv));
+      s->ellv_f32 = true;
+    } else if (s->codec.stage == 5) {
+      GB_TRY(dev_alloc(&s->ellv, rows * 6 * sizeof(double)));
+      ell_vals_kernel<double, 6><<<g, 256>>>(nr, a->rowptr, a->val64,
+          static_cast<double *>(s->ellv));
+    } else {
+      GB_TRY(dev_alloc(&s->ellv, rows * 8 * sizeof(double)));
+      ell_vals_kernel<double, 8><<<g, 256>>>(nr, a->rowptr, a->val64,
+          static_cast<double *>(s->ellv));
+    }
+    GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(cudaDeviceSynchronize());
+  }
+  return GOOSEBERRY_SUCCESS;
+}
+
+// The graph path's two chunk graphs, captured on first use (a solver whose
+// solves run on the chip never needs them).
+int ensure_graphs(gb_cg * s) {
+  if (s->graph[1]) return GOOSEBERRY_SUCCESS;
+  if (!s->cap_stream)
+    GB_CUDA_TRY(cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking));
+  if (!s->graph[0]) GB_TRY(capture_chunk(s, 0));
+  return capture_chunk(s, 1);
+}
+
+// The solve on the chip (cg_resident.cu) for a pattern matrix whose vectors
+// fit the SMs.  A plain-entries solver takes it on the same matrices, reading
+// the CSR arrays, so that both give the same iterates.
+int setup_resident(const gb_csr * a, bool plain, gb_cg * s) {
+  RowPatterns found;
+  ResidentIn in;
+  in.stage = row_stage_for(*a);
+  if (in.stage == 6 || !resident_size_ok(*a)) return GOOSEBERRY_SUCCESS;
+  in.plain = plain;
+  if (plain) GB_TRY(build_row_patterns(*a, &found, nullptr));
+  in.pat = plain ? &found : &s->pat;
+  in.ell8 = s->ell8;
+  in.table = s->codec.table;
+  in.ntable = s->codec.ntable;
+  in.ellv = s->ellv;
+  in.ellv_f32 = s->ellv_f32;
+  in.ellv_width = s->ellv_f32 || in.stage == 7 ? 8 : 6;
+  const int rc = resident_create(*a, in, s->x, &s->resident);
+  free_row_patterns(found);
+  return rc;
+}
+
 // One cooperative launch per solve when every row fits a tile (no long rows)
 // and all CTAs of the grid can be resident at once.  Tiles are dealt to CTAs
 // in contiguous runs of nearly equal rows + nonzeros.
@@ -1288,7 +1367,36 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
     s->a = a;
     s->mode = mode;
     s->n = a->nrows;
-    return mixed_create(a, plain_entries, &s->mixed);
+    GB_TRY(mixed_create(a, plain_entries, &s->mixed));
+    // A system whose FP64 vectors fit the chip is solved there in FP64: its
+    // iterations wait for exchanges and shared memory, not for the bytes that
+    // floats would save, and convergence is still judged on b - A x.
+    if (a->sched64 != GB_SCHED_ROW || a->nnz == 0 || !resident_size_ok(*a))
+      return GOOSEBERRY_SUCCESS;
+    GB_TRY(dev_alloc(&s->x, std::max<size_t>(s->n, 2) * sizeof(double)));
+    if (!plain_entries) {
+      GB_TRY(build_row_codec(*a, &s->codec, nullptr));
+      GB_TRY(build_ell(a, s));
+    }
+    GB_TRY(setup_resident(a, plain_entries, s));
+    if (!s->resident) {  // too wide a band: nothing of this is used
+      free_row_codec(s->codec);
+      free_row_patterns(s->pat);
+      dev_free(s->ell8);
+      dev_free(s->ellv);
+      dev_free(s->x);
+      s->ell8 = nullptr;
+      s->ellv = nullptr;
+      s->x = nullptr;
+      return GOOSEBERRY_SUCCESS;
+    }
+    GB_TRY(dev_alloc(&s->r, s->n * sizeof(double)));
+    GB_TRY(dev_alloc(&s->xsum, s->n * sizeof(double)));
+    GB_TRY(dev_alloc(&s->partial_a, static_cast<size_t>(a->sm_count) * 4 * sizeof(double)));
+    GB_TRY(dev_alloc(&s->ticket, sizeof(unsigned)));
+    GB_CUDA_TRY(cudaMemset(s->ticket, 0, sizeof(unsigned)));
+    return pinned_slot_alloc(sizeof(double), reinterpret_cast<void **>(&s->rr_true_h),
+        reinterpret_cast<void **>(&s->rr_true_d));
   }
   GB_CHECK_INPUT(a->val64 != nullptr, "CG (FP64) needs double values on the matrix");
   s->a = a;
@@ -1309,36 +1417,8 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
     GB_TRY(build_row_codec(*a, &s->codec, nullptr));
     s->use_codec = s->codec.col16 || s->codec.code8 || s->codec.val32;
     entry_bytes = s->codec.entry_bytes();
-    // a pattern matrix: its values (or their codes) in rows of 8, no rowptr
-    if (GB_CG_ELL && a->nnz > 0 && (s->codec.stage == 5 || s->codec.stage == 7)) {
-      GB_TRY(build_row_patterns(*a, &s->pat, nullptr));
-      if (s->pat.code8) {
-        const size_t rows = std::max<size_t>(s->n, 1);
-        const unsigned g = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(
-            (s->n + 255) / 256, static_cast<size_t>(a->sm_count) * 8)));
-        const uint32_t nr = static_cast<uint32_t>(s->n);
-        if (s->codec.code8) {
-          GB_TRY(dev_alloc(&s->ell8, rows * sizeof(uint2)));
-          ell8_codes_kernel<<<g, 256>>>(nr, a->rowptr, s->codec.code8, s->ell8);
-        } else if (s->codec.val32) {
-          GB_TRY(dev_alloc(&s->ellv, rows * 8 * sizeof(float)));
-          ell_vals_kernel<float, 8><<<g, 256>>>(nr, a->rowptr, s->codec.val32,
-              static_cast<float *>(s->ellv));
-          s->ellv_f32 = true;
-        } else if (s->codec.stage == 5) {
-          GB_TRY(dev_alloc(&s->ellv, rows * 6 * sizeof(double)));
-          ell_vals_kernel<double, 6><<<g, 256>>>(nr, a->rowptr, a->val64,
-              static_cast<double *>(s->ellv));
-        } else {
-          GB_TRY(dev_alloc(&s->ellv, rows * 8 * sizeof(double)));
-          ell_vals_kernel<double, 8><<<g, 256>>>(nr, a->rowptr, a->val64,
-              static_cast<double *>(s->ellv));
-        }
-        GB_CUDA_TRY(cudaGetLastError());
-        GB_CUDA_TRY(cudaDeviceSynchronize());
-        entry_bytes = 0;
-      }
-    }
+    if (a->nnz > 0 && GB_CG_ELL) GB_TRY(build_ell(a, s));
+    if (s->ell8 || s->ellv) entry_bytes = 0;
   }
   // evict-first/evict-last hints keep an L2-sized working set (matrix, rowptr,
   // r, both p, Ap, x) resident across iterations; beyond L2 the plain loads win
@@ -1377,11 +1457,8 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
   GB_TRY(pinned_slot_alloc(2 * sizeof(CgStatus), reinterpret_cast<void **>(&s->host_status),
       nullptr));
   if (want_persistent) GB_TRY(setup_persistent(a, s));
-  if (!s->persistent) {
-    GB_CUDA_TRY(cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking));
-    GB_TRY(capture_chunk(s, 0));
-    GB_TRY(capture_chunk(s, 1));
-  }
+  else if (s->sched == GB_SCHED_ROW) GB_TRY(setup_resident(a, plain_entries, s));
+  if (!s->persistent && !s->resident) GB_TRY(ensure_graphs(s));
   return GOOSEBERRY_SUCCESS;
 }
 
@@ -1389,6 +1466,136 @@ bool cancel_requested(const gb_cg * s) {
   return __atomic_load_n(s->cancel_h, __ATOMIC_ACQUIRE) != 0;
 }
 void clear_cancel(gb_cg * s) { __atomic_store_n(s->cancel_h, 0, __ATOMIC_RELEASE); }
+
+// r = b - A x (rows summed in the reference's order) and r.r into *rr, which
+// may be host-mapped; `ticket` is 0 before and after.
+__global__ void __launch_bounds__(kVecBlock) cg_true_residual_kernel(uint32_t n,
+    const uint32_t * __restrict__ rowptr, const uint32_t * __restrict__ rowind,
+    const double * __restrict__ val, const double * __restrict__ b,
+    const double * __restrict__ x, double * __restrict__ r, double * partial, double * rr,
+    unsigned * ticket) {
+  __shared__ double red[32];
+  __shared__ bool last;
+  double acc = 0.0;
+  for (uint32_t i = blockIdx.x * kVecBlock + threadIdx.x; i < n; i += gridDim.x * kVecBlock) {
+    double sum = 0.0;
+    const uint32_t e = __ldg(rowptr + i + 1);
+    for (uint32_t k = __ldg(rowptr + i); k < e; ++k)
+      sum = add_rn(sum, mul_rn(__ldg(val + k), __ldg(x + __ldg(rowind + k))));
+    const double v = b[i] - sum;
+    r[i] = v;
+    acc += v * v;
+  }
+  const double s = block_sum(acc, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (!arrive_last(ticket, &last)) return;
+  __threadfence();
+  const double t = ordered_sum(partial, gridDim.x, red);
+  if (threadIdx.x == 0) {
+    *ticket = 0;
+    *rr = t;
+  }
+}
+
+__global__ void __launch_bounds__(kVecBlock) cg_add_kernel(size_t n, const double * __restrict__ d,
+    double * __restrict__ x) {
+  for (size_t i = blockIdx.x * kVecBlock + threadIdx.x; i < n;
+       i += static_cast<size_t>(gridDim.x) * kVecBlock)
+    x[i] += d[i];
+}
+
+// A solve on the chip.  *done = false: a wait inside it was given up (some
+// other program holds SMs), and the graph path has to run the solve.
+//
+// A GB_CG_MIXED solver's convergence and iteration limit are judged on the
+// true residual b - A x: when the recurrence has met the tolerance, the
+// residual is formed, and while it is still above, A d = b - A x is solved on
+// and x += d (each time one refinement).
+int solve_resident(gb_cg * s, const double * b, double * x, double tol, int tol_relative,
+    size_t niter, double * history, size_t history_len, gb_cg_result_t * res,
+    cudaStream_t stream, bool * done) {
+  *done = false;
+  const bool refine = s->mode == GB_CG_MIXED;
+  double * dhist = nullptr;
+  const size_t cap = niter ? niter : std::max<size_t>(1000, 100 * s->n);  // see start_solve
+  const size_t hl = history ? std::min(history_len, niter ? niter : history_len) : 0;
+  if (hl) GB_TRY(scratch_alloc(reinterpret_cast<void **>(&dhist), hl * sizeof(double), stream));
+  size_t iters = 0, rounds = 0, launches = 0;
+  double bnorm = 0.0, rnorm = 0.0;
+  int status = GB_CG_CANCELLED;
+  bool aborted = false;
+  const double * rhs = b;
+  const auto body = [&]() -> int {
+    while (true) {
+      ResOutcome out;
+      GB_TRY(resident_solve(s->resident, rhs, tol, rounds ? 0 : tol_relative, cap - iters,
+          dhist ? dhist + std::min(iters, hl) : nullptr, hl - std::min(iters, hl), s->cancel_h,
+          s->cancel_d, false, stream, &out));
+      const ResResult & r = out.result;
+      aborted = r.aborted != 0;
+      if (aborted) return GOOSEBERRY_SUCCESS;
+      status = out.cancelled_waiting ? GB_CG_CANCELLED : r.status;
+      launches += out.cancelled_waiting ? 0 : 1;
+      const unsigned g = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(
+          (s->n + kVecBlock - 1) / kVecBlock, static_cast<size_t>(s->a->sm_count) * 4)));
+      if (out.cancelled_waiting) {
+        if (rounds == 0) GB_CUDA_TRY(cudaMemsetAsync(x, 0, s->n * sizeof(double), stream));
+      } else if (rounds == 0) {
+        bnorm = r.bnorm;
+        if (tol_relative) tol *= bnorm;
+        GB_CUDA_TRY(cudaMemcpyAsync(refine ? s->xsum : x, s->x, s->n * sizeof(double),
+            cudaMemcpyDeviceToDevice, stream));
+      } else {
+        cg_add_kernel<<<g, kVecBlock, 0, stream>>>(s->n, s->x, s->xsum);
+        ++launches;
+      }
+      iters += r.iter;
+      rnorm = std::sqrt(r.rr);
+      if (!refine || out.cancelled_waiting || status == GB_CG_NONFINITE || bnorm == 0.0) break;
+      cg_true_residual_kernel<<<g, kVecBlock, 0, stream>>>(static_cast<uint32_t>(s->n),
+          s->a->rowptr, s->a->rowind, s->a->val64, b, s->xsum, s->r, s->partial_a, s->rr_true_d,
+          s->ticket);
+      GB_CUDA_TRY(cudaGetLastError());
+      GB_CUDA_TRY(cudaStreamSynchronize(stream));
+      ++rounds;
+      ++launches;
+      rnorm = std::sqrt(*const_cast<volatile double *>(s->rr_true_h));
+      if (!std::isfinite(rnorm)) status = GB_CG_NONFINITE;
+      else if (status == GB_CG_CONVERGED && rnorm > tol) {
+        status = GB_CG_MAXITER;
+        if (iters < cap) {
+          rhs = s->r;
+          continue;
+        }
+      } else if (status == GB_CG_MAXITER && rnorm <= tol) {
+        status = GB_CG_CONVERGED;
+      }
+      break;
+    }
+    if (refine && launches)
+      GB_CUDA_TRY(cudaMemcpyAsync(x, s->xsum, s->n * sizeof(double), cudaMemcpyDeviceToDevice,
+          stream));
+    if (hl && iters)
+      GB_CUDA_TRY(cudaMemcpyAsync(history, dhist, std::min<size_t>(hl, iters) * sizeof(double),
+          cudaMemcpyDeviceToHost, stream));
+    GB_CUDA_TRY(cudaStreamSynchronize(stream));
+    return GOOSEBERRY_SUCCESS;
+  };
+  const int rc = body();
+  if (dhist) scratch_free(dhist, stream);
+  if (rc != GOOSEBERRY_SUCCESS || aborted) return rc;
+  if (status == GB_CG_CANCELLED) clear_cancel(s);
+  if (res) {
+    res->iterations = iters;
+    res->refinements = rounds;
+    res->rnorm = rnorm;
+    res->bnorm = bnorm;
+    res->status = status;
+    res->kernel_launches = launches;
+  }
+  *done = true;
+  return GOOSEBERRY_SUCCESS;
+}
 
 int start_solve(gb_cg * s, const double * b, double tol, int tol_relative, size_t niter,
     double * dhist, size_t hl, cudaStream_t stream) {
@@ -1414,6 +1621,13 @@ int solve_cg(gb_cg * s, const double * b, double * x, double tol, int tol_relati
     size_t niter, double * history, size_t history_len, gb_cg_result_t * res,
     cudaStream_t stream) {
   if (s->mixed) {
+    if (s->resident) {
+      GB_CHECK_INPUT(b && x, "NULL vector");
+      bool done = false;
+      GB_TRY(solve_resident(s, b, x, tol, tol_relative, niter, history, history_len, res, stream,
+          &done));
+      if (done) return GOOSEBERRY_SUCCESS;
+    }
     const int rc = mixed_solve(s->mixed, b, x, tol, tol_relative, niter, history, history_len,
         res, stream, s->cancel_h);
     if (rc == GOOSEBERRY_SUCCESS && res && res->status == GB_CG_CANCELLED) clear_cancel(s);
@@ -1425,6 +1639,13 @@ int solve_cg(gb_cg * s, const double * b, double * x, double tol, int tol_relati
   if (s->n == 0) {
     if (res) *res = gb_cg_result_t{0, 0, 0.0, 0.0, GB_CG_CONVERGED, 0};
     return GOOSEBERRY_SUCCESS;
+  }
+  if (s->resident) {
+    bool done = false;
+    GB_TRY(solve_resident(s, b, x, tol, tol_relative, niter, history, history_len, res, stream,
+        &done));
+    if (done) return GOOSEBERRY_SUCCESS;
+    GB_TRY(ensure_graphs(s));
   }
   double * dhist = nullptr;
   const size_t hl = history ? std::min(history_len, niter ? niter : history_len) : 0;
@@ -1541,6 +1762,17 @@ int profile_cg(gb_cg * s, const double * b, size_t iterations, double * ms, size
     return GOOSEBERRY_SUCCESS;
   }
   if (nkernels) *nkernels = 2;
+  if (s->resident) {  // the two phases of an iteration, as the solve's kernel times them
+    ResOutcome out;
+    GB_TRY(resident_solve(s->resident, b, 0.0, 0, iterations, nullptr, 0, s->cancel_h,
+        s->cancel_d, true, stream, &out));
+    const double n = 1e6 * std::max<double>(1.0, static_cast<double>(out.result.iter));
+    if (!out.result.aborted) {
+      if (ms && ms_len > 0) ms[0] = static_cast<double>(out.result.ns_a) / n;
+      if (ms && ms_len > 1) ms[1] = static_cast<double>(out.result.ns_b) / n;
+      return GOOSEBERRY_SUCCESS;
+    }
+  }
   GB_TRY(start_solve(s, b, 0.0, 0, 0, nullptr, 0, stream));
   std::vector<cudaEvent_t> ev(3 * iterations);
   for (auto & e : ev) GB_CUDA_TRY(cudaEventCreate(&e));

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_resident.h"
 #include "gb_internal.h"
 #include "spmv_tiles.cuh"
 
@@ -210,6 +211,18 @@ __global__ void codec_pattern_encode_kernel(const uint32_t * __restrict__ rowptr
   }
 }
 
+// key[i] = row i's value codes (bytes 0-6, zero-padded) and pattern (byte 7):
+// equal keys are equal rows, offsets and values.
+__global__ void codec_row_key_kernel(uint32_t n, const uint2 * __restrict__ ell8,
+    const uint8_t * __restrict__ pcode, unsigned long long * __restrict__ key) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint2 w = __ldg(ell8 + i);
+    key[i] = static_cast<unsigned long long>(w.x) |
+             static_cast<unsigned long long>((w.y & 0xffffffu) |
+                                             static_cast<uint32_t>(__ldg(pcode + i)) << 24) << 32;
+  }
+}
+
 int grid_of(const gb_csr & a, size_t items) {
   const size_t want = (items + 255) / 256;
   return static_cast<int>(std::max<size_t>(1, std::min<size_t>(want,
@@ -350,6 +363,77 @@ int build_row_patterns(const gb_csr & a, RowPatterns * out, cudaStream_t s) {
       keys, d_slot, out->off, out->code8, flags);
   if ((rc = read_flag(flags, &bad, s)) != GOOSEBERRY_SUCCESS) return done(rc);
   return done(GOOSEBERRY_SUCCESS);
+}
+
+int build_row_classes(const gb_csr & a, const RowPatterns & pat, const std::vector<int32_t> & off,
+    const uint2 * ell8, const double * table, uint32_t ntable, RowClasses * out,
+    cudaStream_t s) {
+  *out = RowClasses{};
+  const uint32_t n = a.nrows;
+  // the hash set (keys, slot codes, count, flag), then one key per row
+  unsigned char * mem = nullptr;
+  const size_t head = kSetSlots * 8 + kSetSlots + 64;
+  GB_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), head + static_cast<size_t>(n) * 8, s));
+  unsigned long long * keys = reinterpret_cast<unsigned long long *>(mem);
+  uint8_t * d_slot = mem + kSetSlots * 8;
+  unsigned * cnt = reinterpret_cast<unsigned *>(d_slot + kSetSlots);
+  unsigned long long * row_key = reinterpret_cast<unsigned long long *>(mem + head);
+  std::vector<unsigned long long> hk(kSetSlots + 1, kEmpty);
+  std::vector<double> ht(std::max<uint32_t>(ntable, 1));
+  std::vector<ResRowClass> rows;
+  std::vector<uint8_t> slot_code(kSetSlots, 0);
+  int rc = GOOSEBERRY_SUCCESS;
+  const auto body = [&]() -> int {
+    GB_CUDA_TRY(cudaMemcpyAsync(keys, hk.data(), kSetSlots * 8, cudaMemcpyHostToDevice, s));
+    GB_CUDA_TRY(cudaMemsetAsync(cnt, 0, 16, s));
+    codec_row_key_kernel<<<grid_of(a, n), 256, 0, s>>>(n, ell8, pat.code8, row_key);
+    codec_set_kernel<<<grid_of(a, n), 256, 0, s>>>(reinterpret_cast<const double *>(row_key), n,
+        keys, cnt, cnt + 2);
+    GB_CUDA_TRY(cudaGetLastError());
+    unsigned flags[4] = {0, 0, 1, 0};
+    GB_CUDA_TRY(cudaMemcpyAsync(flags, cnt, 16, cudaMemcpyDeviceToHost, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(hk.data(), keys, kSetSlots * 8, cudaMemcpyDeviceToHost, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(ht.data(), table, ntable * 8, cudaMemcpyDeviceToHost, s));
+    GB_CUDA_TRY(cudaStreamSynchronize(s));
+    if (flags[2]) return GOOSEBERRY_SUCCESS;
+    for (unsigned h = 0; h < kSetSlots; ++h) {
+      if (hk[h] == kEmpty) continue;
+      slot_code[h] = static_cast<uint8_t>(rows.size());
+      ResRowClass c{};
+      const uint32_t p = static_cast<uint32_t>(hk[h] >> 56);
+      if (p >= pat.npat) return GOOSEBERRY_SUCCESS;
+      for (int j = 0; j < kPatMax; ++j) c.off[j] = off[p * kPatMax + j];
+      for (int j = 0; j < c.off[kPatMax - 1]; ++j) {
+        const uint32_t v = static_cast<uint32_t>(hk[h] >> (8 * j)) & 0xffu;
+        if (v >= ntable) return GOOSEBERRY_SUCCESS;
+        c.val[j] = ht[v];
+      }
+      rows.push_back(c);
+    }
+    if (rows.empty() || rows.size() != flags[0] || rows.size() > kMaxCodes)
+      return GOOSEBERRY_SUCCESS;
+    GB_TRY(dev_alloc(&out->code8, n));
+    GB_TRY(dev_alloc(&out->rows, rows.size() * sizeof(ResRowClass)));
+    GB_CUDA_TRY(cudaMemcpyAsync(out->rows, rows.data(), rows.size() * sizeof(ResRowClass),
+        cudaMemcpyHostToDevice, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(d_slot, slot_code.data(), kSetSlots, cudaMemcpyHostToDevice, s));
+    codec_encode_kernel<<<grid_of(a, n), 256, 0, s>>>(reinterpret_cast<const double *>(row_key),
+        n, keys, d_slot, out->code8);
+    GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(cudaStreamSynchronize(s));
+    out->count = static_cast<uint32_t>(rows.size());
+    return GOOSEBERRY_SUCCESS;
+  };
+  rc = body();
+  scratch_free(mem, s);
+  if (out->count == 0) free_row_classes(*out);
+  return rc;
+}
+
+void free_row_classes(RowClasses & c) {
+  if (c.code8) dev_free(c.code8);
+  if (c.rows) dev_free(c.rows);
+  c = RowClasses{};
 }
 
 void free_row_patterns(RowPatterns & p) {

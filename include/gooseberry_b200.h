@@ -253,8 +253,18 @@ GOOSEBERRY_API int gb_add_scalar_f32(size_t n, float * v, float s, gb_stream_t s
 
 typedef enum gb_cg_mode {
   GB_CG_F64 = 0,   /* plain FP64 CG, the reference's algorithm             */
-  GB_CG_MIXED = 1  /* FP32 values/vectors inside, FP64 residual refinement  */
+  GB_CG_MIXED = 1  /* FP32 values/vectors inside, FP64 residual refinement;
+                      systems that fit the chip (below) iterate in FP64    */
 } gb_cg_mode_t;
+
+/* On the row schedule, a matrix with at most 7 entries a row and at most 256
+ * distinct column-offset patterns (stencils) whose vectors fit the SMs'
+ * shared memory (up to about 1.08 million rows on 148 SMs, fewer with a wide
+ * band) is solved in one cooperative launch with the vectors on the chip.
+ * Such solves of one process share a device's SMs: each holds as many as it
+ * has CTAs until it ends, and waits for them in order of arrival.  Should a
+ * wait inside a solve exceed 2 s (another program holds SMs), the solve is run
+ * again by the graph-replayed kernels. */
 
 /* OR-ed into the mode of gb_cg_create: run the whole solve as ONE persistent
  * cooperative launch (CTAs own fixed rows; two grid barriers per iteration)
@@ -339,7 +349,8 @@ GOOSEBERRY_API int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned l
  * iterations launch by launch, timing every launch with CUDA events on
  * `stream`.  ms[k] receives the mean duration in milliseconds of kernel k of
  * an iteration (k < nkernels; F64: 0 = SpMV+direction+p.Ap, 1 = x/r update +
- * r.r).  Returns the number of kernels per iteration in *nkernels.  Leaves
+ * r.r; for a solve on the chip the two phases of its one kernel, each with
+ * its exchange between the SMs, as the kernel times them).  Returns the number of kernels per iteration in *nkernels.  Leaves
  * the solver ready for the next gb_cg_solve.  No reference counterpart (the
  * reference only has wall-clock phase timers, src/gooseberry_bin.c:2078-2113).
  */
