@@ -933,8 +933,7 @@ int resident_create(const gb_csr & a, const ResidentIn & in, double * x, Residen
   int src = RES_CSR;
   if (!in.plain) {
     if (in.ell8) {
-      if ((rc = build_row_classes(a, *in.pat, off, in.ell8, in.table, in.ntable,
-               &s->classes, nullptr)) != GOOSEBERRY_SUCCESS)
+      if ((rc = build_row_classes(a, a.val64, &s->classes, nullptr)) != GOOSEBERRY_SUCCESS)
         return fail(rc);
       if (s->classes.code8) {
         src = RES_CLASS;

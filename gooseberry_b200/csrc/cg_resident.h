@@ -17,16 +17,30 @@ struct ResRowClass {
   double val[8];
 };
 
-// Distinct rows of a pattern matrix with coded values, at most 256.
+// The distinct rows of a matrix (rows of at most 7 entries), at most 256.
 struct RowClasses {
   uint8_t * code8 = nullptr;     // [nrows]
   ResRowClass * rows = nullptr;  // [count]
   uint32_t count = 0;
 };
-// `off` is the host copy of pat.off.  Leaves `out` empty past 256 classes.
-int build_row_classes(const gb_csr & a, const RowPatterns & pat, const std::vector<int32_t> & off,
-    const uint2 * ell8, const double * table, uint32_t ntable, RowClasses * out, cudaStream_t s);
+// Leaves `out` empty past 256 classes, or for longer rows.
+int build_row_classes(const gb_csr & a, const double * val, RowClasses * out, cudaStream_t s);
+int build_row_classes(const gb_csr & a, const float * val, RowClasses * out, cudaStream_t s);
 void free_row_classes(RowClasses & c);
+
+// A pattern matrix for plain SpMV (spmv_pattern.cu): its classes, or else its
+// column patterns.
+struct SpmvPattern {
+  RowPatterns pat;
+  RowClasses cls;
+};
+// *out stays null when the matrix has neither.
+int build_spmv_pattern(const gb_csr & a, bool f32, SpmvPattern ** out, cudaStream_t s);
+void free_spmv_pattern(SpmvPattern * p);
+int launch_spmv_pattern(const gb_csr & a, const SpmvPattern & p, const double * x, double * y,
+    uint32_t stride, cudaStream_t s);
+int launch_spmv_pattern(const gb_csr & a, const SpmvPattern & p, const float * x, float * y,
+    uint32_t stride, cudaStream_t s);
 
 // What the solve kernel reports, in pinned host memory.
 struct ResResult {

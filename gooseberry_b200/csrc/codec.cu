@@ -211,15 +211,98 @@ __global__ void codec_pattern_encode_kernel(const uint32_t * __restrict__ rowptr
   }
 }
 
-// key[i] = row i's value codes (bytes 0-6, zero-padded) and pattern (byte 7):
-// equal keys are equal rows, offsets and values.
-__global__ void codec_row_key_kernel(uint32_t n, const uint2 * __restrict__ ell8,
-    const uint8_t * __restrict__ pcode, unsigned long long * __restrict__ key) {
+// ---- row classes: whole rows, offsets and values ---------------------------------
+
+__device__ __forceinline__ unsigned long long value_bits(double v) {
+  return static_cast<unsigned long long>(__double_as_longlong(v));
+}
+__device__ __forceinline__ unsigned long long value_bits(float v) {
+  return static_cast<unsigned long long>(__float_as_uint(v));
+}
+
+// Hash of a row's column offsets and the bits of its values.
+template <typename T>
+__device__ __forceinline__ unsigned long long row_hash(const uint32_t * __restrict__ rowind,
+    const T * __restrict__ val, uint32_t b, uint32_t e, uint32_t row) {
+  unsigned long long h = pattern_hash(rowind, b, e, row);
+  for (uint32_t k = b; k < e; ++k) {
+    h ^= value_bits(__ldg(val + k)) + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
+    h *= 0xff51afd7ed558ccdull;
+    h ^= h >> 33;
+  }
+  return h == kEmpty ? h ^ 1ull : h;
+}
+
+// Distinct rows into the hash set, with a row holding each; *bad = 1 past
+// kMaxCodes rows.  (The first rows are tried alone: most matrices without
+// repeating rows are turned away by them.)
+template <typename T>
+__global__ void codec_class_set_kernel(const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const T * __restrict__ val, uint32_t n,
+    unsigned long long * keys, uint32_t * rep, unsigned * count, unsigned * bad) {
+  if (*reinterpret_cast<volatile unsigned *>(bad)) return;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint2 w = __ldg(ell8 + i);
-    key[i] = static_cast<unsigned long long>(w.x) |
-             static_cast<unsigned long long>((w.y & 0xffffffu) |
-                                             static_cast<uint32_t>(__ldg(pcode + i)) << 24) << 32;
+    if ((i & 255u) == 0 && *reinterpret_cast<volatile unsigned *>(bad)) return;
+    const uint32_t b = __ldg(rowptr + i), e = __ldg(rowptr + i + 1);
+    const unsigned long long h0 = row_hash(rowind, val, b, e, i);
+    unsigned h = slot_of(h0);
+    bool placed = false;
+    for (unsigned probe = 0; probe < kSetSlots && !placed; ++probe, h = (h + 1) & (kSetSlots - 1)) {
+      unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(keys + h);
+      if (cur == kEmpty) {
+        cur = atomicCAS(keys + h, kEmpty, h0);
+        if (cur == kEmpty) {
+          rep[h] = i;
+          if (atomicAdd(count, 1u) >= kMaxCodes) atomicExch(bad, 1u);
+          placed = true;
+        }
+      }
+      if (cur == h0) placed = true;
+    }
+    if (!placed) {
+      atomicExch(bad, 1u);
+      return;
+    }
+  }
+}
+
+template <typename T>
+__global__ void codec_class_table_kernel(const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const T * __restrict__ val,
+    const unsigned long long * __restrict__ keys, const uint32_t * __restrict__ rep,
+    const uint8_t * __restrict__ slot_code, ResRowClass * __restrict__ rows) {
+  const unsigned h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= kSetSlots || keys[h] == kEmpty) return;
+  const uint32_t row = rep[h], b = rowptr[row], e = rowptr[row + 1];
+  ResRowClass & c = rows[slot_code[h]];
+  for (int j = 0; j < kPatMax; ++j) {
+    const bool in = j + 1 < kPatMax && b + j < e;
+    c.off[j] = in ? static_cast<int32_t>(rowind[b + j] - row) : 0;
+    c.val[j] = in ? static_cast<double>(val[b + j]) : 0.0;
+  }
+  c.off[kPatMax - 1] = static_cast<int32_t>(e - b);
+}
+
+// code8[i] = class of row i; every row is compared with its class, bit for bit
+// (*bad = 1 on a mismatch, which only a hash collision could cause).
+template <typename T>
+__global__ void codec_class_encode_kernel(const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const T * __restrict__ val, uint32_t n,
+    const unsigned long long * __restrict__ keys, const uint8_t * __restrict__ slot_code,
+    const ResRowClass * __restrict__ rows, uint8_t * __restrict__ code8, unsigned * bad) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t b = __ldg(rowptr + i), e = __ldg(rowptr + i + 1);
+    const unsigned long long h0 = row_hash(rowind, val, b, e, i);
+    unsigned h = slot_of(h0);
+    for (unsigned probe = 0; probe < kSetSlots; ++probe, h = (h + 1) & (kSetSlots - 1))
+      if (__ldg(keys + h) == h0) break;
+    const uint32_t c = __ldg(slot_code + h);
+    code8[i] = static_cast<uint8_t>(c);
+    bool same = e - b == static_cast<uint32_t>(rows[c].off[kPatMax - 1]);
+    for (uint32_t k = b; same && k < e; ++k)
+      same = __ldg(rowind + k) == i + static_cast<uint32_t>(rows[c].off[k - b]) &&
+             value_bits(__ldg(val + k)) == value_bits(static_cast<T>(rows[c].val[k - b]));
+    if (!same) atomicExch(bad, 1u);
   }
 }
 
@@ -365,69 +448,65 @@ int build_row_patterns(const gb_csr & a, RowPatterns * out, cudaStream_t s) {
   return done(GOOSEBERRY_SUCCESS);
 }
 
-int build_row_classes(const gb_csr & a, const RowPatterns & pat, const std::vector<int32_t> & off,
-    const uint2 * ell8, const double * table, uint32_t ntable, RowClasses * out,
-    cudaStream_t s) {
+namespace {
+template <typename T>
+int build_classes(const gb_csr & a, const T * val, RowClasses * out, cudaStream_t s) {
   *out = RowClasses{};
   const uint32_t n = a.nrows;
-  // the hash set (keys, slot codes, count, flag), then one key per row
-  unsigned char * mem = nullptr;
-  const size_t head = kSetSlots * 8 + kSetSlots + 64;
-  GB_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), head + static_cast<size_t>(n) * 8, s));
-  unsigned long long * keys = reinterpret_cast<unsigned long long *>(mem);
-  uint8_t * d_slot = mem + kSetSlots * 8;
+  if (n == 0 || !val || a.plan.max_row >= static_cast<uint32_t>(kPatMax)) return GOOSEBERRY_SUCCESS;
+  // keys, representative rows, slot codes, count and flag
+  unsigned long long * keys = nullptr;
+  GB_TRY(scratch_alloc(reinterpret_cast<void **>(&keys), kSetSlots * 13 + 64, s));
+  uint32_t * rep = reinterpret_cast<uint32_t *>(keys + kSetSlots);
+  uint8_t * d_slot = reinterpret_cast<uint8_t *>(rep + kSetSlots);
   unsigned * cnt = reinterpret_cast<unsigned *>(d_slot + kSetSlots);
-  unsigned long long * row_key = reinterpret_cast<unsigned long long *>(mem + head);
-  std::vector<unsigned long long> hk(kSetSlots + 1, kEmpty);
-  std::vector<double> ht(std::max<uint32_t>(ntable, 1));
-  std::vector<ResRowClass> rows;
+  std::vector<unsigned long long> hk(kSetSlots, kEmpty);
   std::vector<uint8_t> slot_code(kSetSlots, 0);
-  int rc = GOOSEBERRY_SUCCESS;
+  bool good = false;
   const auto body = [&]() -> int {
     GB_CUDA_TRY(cudaMemcpyAsync(keys, hk.data(), kSetSlots * 8, cudaMemcpyHostToDevice, s));
     GB_CUDA_TRY(cudaMemsetAsync(cnt, 0, 16, s));
-    codec_row_key_kernel<<<grid_of(a, n), 256, 0, s>>>(n, ell8, pat.code8, row_key);
-    codec_set_kernel<<<grid_of(a, n), 256, 0, s>>>(reinterpret_cast<const double *>(row_key), n,
-        keys, cnt, cnt + 2);
+    codec_class_set_kernel<T><<<grid_of(a, std::min(n, 16384u)), 256, 0, s>>>(a.rowptr, a.rowind,
+        val, std::min(n, 16384u), keys, rep, cnt, cnt + 2);
+    if (n > 16384u)
+      codec_class_set_kernel<T><<<grid_of(a, n), 256, 0, s>>>(a.rowptr, a.rowind, val, n, keys,
+          rep, cnt, cnt + 2);
     GB_CUDA_TRY(cudaGetLastError());
     unsigned flags[4] = {0, 0, 1, 0};
     GB_CUDA_TRY(cudaMemcpyAsync(flags, cnt, 16, cudaMemcpyDeviceToHost, s));
     GB_CUDA_TRY(cudaMemcpyAsync(hk.data(), keys, kSetSlots * 8, cudaMemcpyDeviceToHost, s));
-    GB_CUDA_TRY(cudaMemcpyAsync(ht.data(), table, ntable * 8, cudaMemcpyDeviceToHost, s));
     GB_CUDA_TRY(cudaStreamSynchronize(s));
     if (flags[2]) return GOOSEBERRY_SUCCESS;
-    for (unsigned h = 0; h < kSetSlots; ++h) {
-      if (hk[h] == kEmpty) continue;
-      slot_code[h] = static_cast<uint8_t>(rows.size());
-      ResRowClass c{};
-      const uint32_t p = static_cast<uint32_t>(hk[h] >> 56);
-      if (p >= pat.npat) return GOOSEBERRY_SUCCESS;
-      for (int j = 0; j < kPatMax; ++j) c.off[j] = off[p * kPatMax + j];
-      for (int j = 0; j < c.off[kPatMax - 1]; ++j) {
-        const uint32_t v = static_cast<uint32_t>(hk[h] >> (8 * j)) & 0xffu;
-        if (v >= ntable) return GOOSEBERRY_SUCCESS;
-        c.val[j] = ht[v];
-      }
-      rows.push_back(c);
-    }
-    if (rows.empty() || rows.size() != flags[0] || rows.size() > kMaxCodes)
-      return GOOSEBERRY_SUCCESS;
+    uint32_t count = 0;
+    for (unsigned h = 0; h < kSetSlots; ++h)
+      if (hk[h] != kEmpty) slot_code[h] = static_cast<uint8_t>(count++);
+    if (count == 0 || count != flags[0] || count > kMaxCodes) return GOOSEBERRY_SUCCESS;
     GB_TRY(dev_alloc(&out->code8, n));
-    GB_TRY(dev_alloc(&out->rows, rows.size() * sizeof(ResRowClass)));
-    GB_CUDA_TRY(cudaMemcpyAsync(out->rows, rows.data(), rows.size() * sizeof(ResRowClass),
-        cudaMemcpyHostToDevice, s));
+    GB_TRY(dev_alloc(&out->rows, count * sizeof(ResRowClass)));
+    out->count = count;
     GB_CUDA_TRY(cudaMemcpyAsync(d_slot, slot_code.data(), kSetSlots, cudaMemcpyHostToDevice, s));
-    codec_encode_kernel<<<grid_of(a, n), 256, 0, s>>>(reinterpret_cast<const double *>(row_key),
-        n, keys, d_slot, out->code8);
+    codec_class_table_kernel<T><<<kSetSlots / 256, 256, 0, s>>>(a.rowptr, a.rowind, val, keys, rep,
+        d_slot, out->rows);
+    codec_class_encode_kernel<T><<<grid_of(a, n), 256, 0, s>>>(a.rowptr, a.rowind, val, n, keys,
+        d_slot, out->rows, out->code8, cnt + 2);
     GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(cudaMemcpyAsync(flags, cnt, 16, cudaMemcpyDeviceToHost, s));
     GB_CUDA_TRY(cudaStreamSynchronize(s));
-    out->count = static_cast<uint32_t>(rows.size());
+    good = flags[2] == 0;
     return GOOSEBERRY_SUCCESS;
   };
-  rc = body();
-  scratch_free(mem, s);
-  if (out->count == 0) free_row_classes(*out);
+  const int rc = body();
+  scratch_free(keys, s);
+  if (!good) free_row_classes(*out);
   return rc;
+}
+}  // namespace
+
+int build_row_classes(const gb_csr & a, const double * val, RowClasses * out, cudaStream_t s) {
+  return build_classes(a, val, out, s);
+}
+int build_row_classes(const gb_csr & a, const float * val, RowClasses * out, cudaStream_t s) {
+  return build_classes(a, val, out, s);
 }
 
 void free_row_classes(RowClasses & c) {

@@ -130,6 +130,8 @@ uint32_t seg_max_warps(int sm_count);
 int upload_plan(Plan & plan, cudaStream_t stream);
 void free_plan(Plan & plan);
 
+struct SpmvPattern;
+
 }  // namespace gb
 
 // ---- the opaque handles -----------------------------------------------------
@@ -150,6 +152,10 @@ struct gb_csr {
   int sched64 = GB_SCHED_AUTO;  // resolved schedule (never AUTO after create)
   int sched32 = GB_SCHED_AUTO;
   int sm_count = 0;
+  // the row schedule's compressed forms (spmv_pattern.cu), where the autotuner
+  // found them faster
+  gb::SpmvPattern * pat64 = nullptr;
+  gb::SpmvPattern * pat32 = nullptr;
 };
 
 namespace gb {

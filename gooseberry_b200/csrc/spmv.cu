@@ -15,6 +15,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cg_resident.h"
 #include "gb_internal.h"
 #include "spmv_seg.cuh"
 #include "spmv_tiles.cuh"
@@ -597,6 +598,8 @@ int launch_sched(const gb_csr & a, int sched, const V * val, const Gather & g,
 int launch_spmv_f64(const gb_csr & a, int sched, const double * x, double * y,
     uint32_t stride, cudaStream_t stream) {
   GB_CHECK_INPUT(a.val64 != nullptr, "matrix holds no double values");
+  if (sched == GB_SCHED_ROW && a.pat64)
+    return launch_spmv_pattern(a, *a.pat64, x, y, stride, stream);
   GatherPlain<double> g{x};
   OutStore<double, double> o{y, stride};
   return launch_sched<double, double>(a, sched, a.val64, g, o, stream);
@@ -605,6 +608,8 @@ int launch_spmv_f64(const gb_csr & a, int sched, const double * x, double * y,
 int launch_spmv_f32(const gb_csr & a, int sched, const float * x, float * y,
     uint32_t stride, cudaStream_t stream) {
   GB_CHECK_INPUT(a.val32 != nullptr, "matrix holds no float values");
+  if (sched == GB_SCHED_ROW && a.pat32)
+    return launch_spmv_pattern(a, *a.pat32, x, y, stride, stream);
   GatherPlain<float> g{x};
   OutStore<float, float> o{y, stride};
   return launch_sched<float, float>(a, sched, a.val32, g, o, stream);
@@ -647,6 +652,7 @@ struct TuneKey {
 struct TuneChoice {
   int sched;
   uint32_t tile_items;
+  bool pattern = false;  // the row schedule over row patterns
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneChoice> g_tune_cache;
@@ -714,7 +720,18 @@ int ensure_seg_plan(gb_csr & a, cudaStream_t stream) {
   return rc;
 }
 
+// Drop a width's compressed form (work that uses it may still run).
+void drop_pattern(gb_csr & a, unsigned width) {
+  SpmvPattern *& p = width == GB_CSR_VALUES_F32 ? a.pat32 : a.pat64;
+  if (!p) return;
+  cudaDeviceSynchronize();
+  free_spmv_pattern(p);
+  p = nullptr;
+}
+
 int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
+  SpmvPattern *& pattern = width == GB_CSR_VALUES_F32 ? a.pat32 : a.pat64;
+  drop_pattern(a, width);
   const TuneKey key = make_key(a, width);
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -723,7 +740,10 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
       GB_TRY(rebuild_plan(a, it->second.tile_items, stream));
       if (it->second.sched == GB_SCHED_SEG) GB_TRY(ensure_seg_plan(a, stream));
       (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = it->second.sched;
-      return GOOSEBERRY_SUCCESS;
+      // (a matrix of this shape without patterns keeps the plain row schedule)
+      return it->second.pattern
+                 ? build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &pattern, stream)
+                 : GOOSEBERRY_SUCCESS;
     }
   }
   const size_t xb = static_cast<size_t>(a.ncols) * (width == GB_CSR_VALUES_F32 ? 4 : 8);
@@ -741,10 +761,23 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   struct Cand {
     uint32_t tile;
     int sched;
+    bool pattern = false;
   };
   std::vector<Cand> cands;
   const bool short_rows = a.plan.p99 <= 64 && a.plan.max_row <= 4096;
   if (short_rows) cands.push_back({1024, GB_SCHED_ROW});
+  SpmvPattern * trial = nullptr;
+  if (short_rows) {
+    const int prc = build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &trial, stream);
+    if (prc != GOOSEBERRY_SUCCESS) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      dev_free(x);
+      dev_free(y);
+      return prc;
+    }
+    if (trial) cands.push_back({1024, GB_SCHED_ROW, true});
+  }
   for (uint32_t t : {128u, 256u, 512u}) cands.push_back({t, GB_SCHED_WTILE});
   cands.push_back({static_cast<uint32_t>(32 * kWmKt), GB_SCHED_WMERGE});
   const void * vals = width == GB_CSR_VALUES_F32 ? static_cast<const void *>(a.val32)
@@ -761,6 +794,7 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   TuneChoice choice{default_schedule(a.plan), a.plan.tile_items};
   int rc = GOOSEBERRY_SUCCESS;
   for (const Cand & cd : cands) {
+    pattern = cd.pattern ? trial : nullptr;
     rc = rebuild_plan(a, cd.tile, stream);
     if (rc == GOOSEBERRY_SUCCESS && cd.sched == GB_SCHED_SEG) rc = ensure_seg_plan(a, stream);
     if (rc != GOOSEBERRY_SUCCESS) break;
@@ -790,7 +824,7 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
       cudaEventElapsedTime(&ms, e0, e1);
       if (ms < best) {
         best = ms;
-        choice = TuneChoice{s, ti};
+        choice = TuneChoice{s, ti, cd.pattern};
       }
     }
     if (rc != GOOSEBERRY_SUCCESS) break;
@@ -799,6 +833,11 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   cudaEventDestroy(e1);
   dev_free(x);
   dev_free(y);
+  pattern = rc == GOOSEBERRY_SUCCESS && choice.pattern ? trial : nullptr;
+  if (trial && !pattern) {
+    cudaStreamSynchronize(stream);
+    free_spmv_pattern(trial);
+  }
   GB_TRY(rc);
   GB_TRY(rebuild_plan(a, choice.tile_items, stream));
   (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = choice.sched;
@@ -830,7 +869,10 @@ void release(gb_csr * a) {
   if (!a) return;
   // uploads may still be in flight on the creating stream (a creation that
   // failed part-way), and dev_free releases on the pool's own stream
-  if (a->own_rowptr || a->own_rowind || a->own_val64 || a->own_val32) cudaDeviceSynchronize();
+  if (a->own_rowptr || a->own_rowind || a->own_val64 || a->own_val32 || a->pat64 || a->pat32)
+    cudaDeviceSynchronize();
+  gb::free_spmv_pattern(a->pat64);
+  gb::free_spmv_pattern(a->pat32);
   gb::free_plan(a->plan);
   if (a->own_rowptr) dev_free(a->own_rowptr);
   if (a->own_rowind) dev_free(a->own_rowind);
@@ -1025,6 +1067,7 @@ int gb_csr_set_schedule(gb_csr_t * a, unsigned value_width, int schedule,
   GB_CHECK_INPUT(schedule != GB_SCHED_WMERGE ||
                      (tile_items ? tile_items : a->plan.tile_items) <= wm_max,
       "per-warp merge tiles need tile_items <= %u", wm_max);
+  gb::drop_pattern(*a, value_width);
   if (tile_items) GB_TRY(gb::rebuild_plan(*a, tile_items, nullptr));
   if (schedule == GB_SCHED_SEG) GB_TRY(gb::ensure_seg_plan(*a, nullptr));
   const int s = schedule == GB_SCHED_AUTO ? gb::default_schedule(a->plan) : schedule;

@@ -134,7 +134,10 @@ GOOSEBERRY_API int gb_csr_get_info(const gb_csr_t * a, gb_csr_info_t * info);
 GOOSEBERRY_API int gb_csr_set_schedule(gb_csr_t * a, unsigned value_width, int schedule,
     uint32_t tile_items);
 
-/* Time every candidate schedule on this matrix and keep the fastest; the
+/* Time every candidate schedule on this matrix and keep the fastest (for a
+ * matrix with at most 7 entries a row that repeats at most 256 rows, or lists
+ * of column offsets, also the row schedule over a compressed copy with its
+ * results, reported as GB_SCHED_ROW; gb_csr_set_schedule drops it); the
  * choice is cached per process under a key of (row-length quantiles, nrows,
  * nnz, value width) so equal-shaped matrices skip the timing.  Synchronous. */
 GOOSEBERRY_API int gb_csr_autotune(gb_csr_t * a, unsigned value_width, gb_stream_t stream);
