@@ -3,14 +3,14 @@
 //
 // B is column-major (B[j * ncols + c], the reference's layout), C row-major
 // (C[i * k + j]).  One thread per row (grid-stride): the row's first
-// kSpmmStage (or, when every row fits, 5) indices and values are loaded once
-// into registers, then for each column j (two columns at a time on 5-entry
-// rows) all of the row's gathers from those columns of B are issued before any
-// is used, and C[i * k + j] is written.  Each element is summed k ascending
-// with unfused multiply and add, exactly like the reference's inner loop, so C
-// is bit-identical to blas_spmult's.  Against one SpMV per column, A's indices
-// and values leave memory once instead of k times and the product is one
-// launch; few registers per thread keep many rows in flight.  Matrices with
+// kSpmmStage (or, when every row fits, 5 or 7) indices and values are loaded
+// once into registers, then for each group of up to four columns all of the
+// row's gathers from those columns of B are issued before any is used, and the
+// group's entries of C are written, where they fill a 32-byte sector, in one
+// store.  Each element is summed k ascending with unfused multiply and add,
+// exactly like the reference's inner loop, so C is bit-identical to
+// blas_spmult's.  Against one SpMV per column, A's indices and values leave
+// memory once instead of k times and the product is one launch.  Matrices with
 // rows too long for one thread keep the per-column SpMV.
 #include <algorithm>
 
@@ -22,23 +22,38 @@ namespace {
 
 constexpr int kSpmmBlock = 256;
 constexpr int kSpmmStage = 8;  // a row's entries held in registers (longer rows: tail loop)
-// Rows of at most 5 entries (2D stencils) take a 5-entry stage, two columns of
-// B at a time (both columns' gathers in flight together) and three CTAs per
-// SM (80 registers, no spills): on the 1024^2 Laplacian with k = 8, 82.9 ->
-// 66.1 us.  (The 5-entry stage one column at a time: 104.9 us; pairs at the
-// default occupancy: 76.8 us.)  Longer rows keep the 8-entry stage, one column
-// at a time.
-#ifndef GB_SPMM_PAIRS
-#define GB_SPMM_PAIRS 1
-#endif
-#ifndef GB_SPMM_MIN_BLOCKS
-#define GB_SPMM_MIN_BLOCKS 3
-#endif
 
-template <typename T, int STAGE>
-__global__ void __launch_bounds__(kSpmmBlock, STAGE <= 5 ? GB_SPMM_MIN_BLOCKS : 4) spmm_rows_kernel(uint32_t nrows, uint32_t ncols,
-    uint32_t k, const uint32_t * __restrict__ rowptr, const uint32_t * __restrict__ rowind,
-    const T * __restrict__ val, const T * __restrict__ b, T * __restrict__ c) {
+// N values to consecutive addresses p, p + 1, ...; `wide`: p is aligned to
+// all of them
+template <typename T, int N>
+__device__ __forceinline__ void store_run(T * p, const T (&v)[N], bool wide) {
+  if constexpr (N == 4 && sizeof(T) == 8) {
+    if (wide) {
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]),
+                   "d"(v[2]), "d"(v[3])
+                   : "memory");
+      return;
+    }
+  } else if constexpr (N == 4 && sizeof(T) == 4) {
+    if (wide) {
+      *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+      return;
+    }
+  } else if constexpr (N == 2 && sizeof(T) == 8) {
+    if (wide) {
+      *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+      return;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) p[q] = v[q];
+}
+
+template <typename T, int STAGE, int COLS, int MINB>
+__global__ void __launch_bounds__(kSpmmBlock, MINB) spmm_rows_kernel(
+    uint32_t nrows, uint32_t ncols, uint32_t k, const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const T * __restrict__ val, const T * __restrict__ b,
+    T * __restrict__ c, bool wide) {
   const uint32_t cmax = ncols - 1;
   for (uint32_t i = blockIdx.x * kSpmmBlock + threadIdx.x; i < nrows;
        i += gridDim.x * kSpmmBlock) {
@@ -53,32 +68,30 @@ __global__ void __launch_bounds__(kSpmmBlock, STAGE <= 5 ? GB_SPMM_MIN_BLOCKS : 
       }
     T * crow = c + static_cast<size_t>(i) * k;
     uint32_t j = 0;
-    // two columns at a time: both columns' gathers are in flight together
-    if constexpr (STAGE <= 5 && GB_SPMM_PAIRS) for (; j + 2 <= k; j += 2) {
+    if constexpr (COLS > 1) for (; j + COLS <= k; j += COLS) {
       const T * bj = b + static_cast<size_t>(j) * ncols;
-      const T * bj1 = bj + ncols;
-      T x[STAGE], x1[STAGE];
+      T x[COLS][STAGE];
 #pragma unroll
-      for (int s = 0; s < STAGE; ++s)
-        if (rb + s < re) {
-          x[s] = __ldg(bj + col[s]);
-          x1[s] = __ldg(bj1 + col[s]);
-        }
-      T acc = T(0), acc1 = T(0);
+      for (int q = 0; q < COLS; ++q)
 #pragma unroll
-      for (int s = 0; s < STAGE; ++s)
-        if (rb + s < re) {
-          acc = add_rn(acc, mul_rn(w[s], x[s]));
-          acc1 = add_rn(acc1, mul_rn(w[s], x1[s]));
-        }
+        for (int s = 0; s < STAGE; ++s)
+          if (rb + s < re) x[q][s] = __ldg(bj + q * static_cast<size_t>(ncols) + col[s]);
+      T acc[COLS];
+#pragma unroll
+      for (int q = 0; q < COLS; ++q) {
+        acc[q] = T(0);
+#pragma unroll
+        for (int s = 0; s < STAGE; ++s)
+          if (rb + s < re) acc[q] = add_rn(acc[q], mul_rn(w[s], x[q][s]));
+      }
       for (uint32_t t = rb + STAGE; t < re; ++t) {  // long-row tail
         const uint32_t ct = min(__ldg(rowind + t), cmax);
         const T wt = __ldg(val + t);
-        acc = add_rn(acc, mul_rn(wt, __ldg(bj + ct)));
-        acc1 = add_rn(acc1, mul_rn(wt, __ldg(bj1 + ct)));
+#pragma unroll
+        for (int q = 0; q < COLS; ++q)
+          acc[q] = add_rn(acc[q], mul_rn(wt, __ldg(bj + static_cast<size_t>(q) * ncols + ct)));
       }
-      crow[j] = acc;
-      crow[j + 1] = acc1;
+      store_run<T, COLS>(crow + j, acc, wide);
     }
     for (; j < k; ++j) {
       const T * bj = b + static_cast<size_t>(j) * ncols;
@@ -113,9 +126,24 @@ int launch_spmm_fused(const gb_csr & a, uint32_t k, const T * vals, const T * b,
   GB_TRY(sm_count_of_current_device(&sms));
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(
       (a.nrows + kSpmmBlock - 1) / kSpmmBlock, static_cast<uint32_t>(sms) * 8));
-  auto kern = a.plan.max_row <= 5 ? spmm_rows_kernel<T, 5> : spmm_rows_kernel<T, kSpmmStage>;
+  // Columns at a time (us, one column or a pair at a time -> four): 1024^2
+  // Laplacian, k = 8 62 -> 54; 700^2, k = 16 69 -> 47; 100^3, k = 8 84 -> 66, k =
+  // 16 176 -> 111.  With fewer than four columns a pair (5 entries: k = 2 27 us,
+  // where the four-column form takes 39), or one (7 entries: k = 3 29 us, 40).
+  // Two CTAs an SM, so that the 20 or 28 gathers in flight have registers:
+  // at three the compiler spills (95 us for the first).
+  uint32_t cols = 1;
+  auto kern = spmm_rows_kernel<T, kSpmmStage, 1, 4>;
+  if (a.plan.max_row <= 5) {
+    cols = k >= 4 ? 4 : 2;
+    kern = k >= 4 ? spmm_rows_kernel<T, 5, 4, 2> : spmm_rows_kernel<T, 5, 2, 3>;
+  } else if (a.plan.max_row <= 7 && k >= 4) {
+    cols = 4;
+    kern = spmm_rows_kernel<T, 7, 4, 2>;
+  }
+  const bool wide = k % cols == 0 && reinterpret_cast<uintptr_t>(c) % (cols * sizeof(T)) == 0;
   kern<<<grid, kSpmmBlock, 0, stream>>>(a.nrows, std::max<uint32_t>(a.ncols, 1), k, a.rowptr,
-      a.rowind, vals, b, c);
+      a.rowind, vals, b, c, wide);
   GB_CUDA_TRY(cudaGetLastError());
   return GOOSEBERRY_SUCCESS;
 }
