@@ -65,7 +65,7 @@ int vec_op(ind_t n, T * val, T s, bool add) {
   GB_TRY(rc);
   DevBuf d;
   GB_TRY(gb::dev_alloc(&d.p, n * sizeof(T)));
-  GB_CUDA_TRY(cudaMemcpyAsync(d.p, val, n * sizeof(T), cudaMemcpyHostToDevice, st));
+  GB_TRY(gb::upload(d.p, val, n * sizeof(T), st));
   if (sizeof(T) == 8) {
     rc = add ? gb::launch_add_scalar_f64(n, static_cast<double *>(d.p), s, st)
              : gb::launch_scale_f64(n, static_cast<double *>(d.p), s, st);
@@ -114,7 +114,7 @@ int spmult_impl(dim_t anrows, dim_t ancols, dim_t bncols, const ind_t * rowptr,
   const size_t csz = static_cast<size_t>(anrows) * bncols;
   GB_TRY(gb::dev_alloc(&db.p, std::max<size_t>(bsz, 1) * sizeof(T)));
   GB_TRY(gb::dev_alloc(&dc.p, csz * sizeof(T)));
-  if (bsz) GB_CUDA_TRY(cudaMemcpyAsync(db.p, bcolval, bsz * sizeof(T), cudaMemcpyHostToDevice, st));
+  if (bsz) GB_TRY(gb::upload(db.p, bcolval, bsz * sizeof(T), st));
   bool fused = false;
   GB_TRY(gb::launch_spmm_fused<T>(*g.a, bncols,
       f64 ? reinterpret_cast<const T *>(g.a->val64) : reinterpret_cast<const T *>(g.a->val32),
@@ -167,11 +167,7 @@ int cgd_f64(dim_t n, const ind_t * rowptr, const dim_t * rowind, const double * 
   gb_cg_result_t res{};
   rc = gb::dev_alloc(&db.p, n * sizeof(double));
   if (rc == GOOSEBERRY_SUCCESS) rc = gb::dev_alloc(&dx.p, n * sizeof(double));
-  if (rc == GOOSEBERRY_SUCCESS &&
-      cudaMemcpyAsync(db.p, b, n * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess) {
-    gb::set_error("CG buffers: %s", cudaGetErrorString(cudaGetLastError()));
-    rc = GOOSEBERRY_ERROR_UNKNOWN;
-  }
+  if (rc == GOOSEBERRY_SUCCESS) rc = gb::upload(db.p, b, n * sizeof(double), st);
   if (rc == GOOSEBERRY_SUCCESS)
     rc = gb_cg_solve(s, static_cast<const double *>(db.p), static_cast<double *>(dx.p), error,
         0, niter, history, history_len, &res, st);

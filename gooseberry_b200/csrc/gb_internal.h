@@ -211,6 +211,9 @@ void dev_free(void * p);
 // that uses it can still run.
 int pinned_slot_alloc(size_t bytes, void ** host, void ** dev);
 void pinned_slot_free(void * host);
+// Copy host memory to the current device on stream `s`; the source may be
+// reused on return, as after a pageable cudaMemcpyAsync.
+int upload(void * dst, const void * src, size_t bytes, cudaStream_t s);
 // Raise a kernel's dynamic shared-memory limit on the current device to at
 // least `bytes` (above the 48 KiB default).  Never lowers it: a kernel that is
 // launched, or captured in graphs, at several sizes keeps the largest limit

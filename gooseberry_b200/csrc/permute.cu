@@ -830,8 +830,7 @@ int check_rowptr(uint32_t n, const uint32_t * rowptr, uint32_t * max_row) {
 template <typename T>
 int upload(gb::ScratchSet & sc, T ** d, const T * h, size_t count, cudaStream_t s) {
   GB_TRY(sc.get(d, count));
-  if (count && h)
-    GB_CUDA_TRY(cudaMemcpyAsync(*d, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
+  if (count && h) GB_TRY(gb::upload(*d, h, count * sizeof(T), s));
   return GOOSEBERRY_SUCCESS;
 }
 

@@ -1,5 +1,7 @@
 // runtime.cpp -- error state, device queries and the stream-ordered scratch
 // pool of libgooseberry_b200.
+#include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -7,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "gb_internal.h"
@@ -174,6 +177,109 @@ void pinned_slot_free(void * host) {
   if (!host) return;
   std::lock_guard<std::mutex> lock(g_slot_mu);
   g_slot_free.push_back(host);
+}
+
+// ---- uploads of pageable memory ---------------------------------------------------
+//
+// The driver stages a pageable copy through one thread, at 10-12 GB/s; PCIe
+// takes 50.  Here several threads copy pieces into pinned slots, each piece
+// sent as soon as it is there.  Pieces are 1 MiB and every thread alternates
+// between two slots: 16 MiB of pinned memory per device, kept for the life of
+// the process and used by one upload at a time (another one meanwhile takes the
+// driver's path).  From 24 MiB up: below, starting the threads (0.3 ms) takes
+// what they save (19 MB of CSR arrays: 1.58 ms by the driver, 1.75 so; 196 MB:
+// 18.8 and 7.2).
+namespace {
+constexpr size_t kUpPiece = 1 << 20;
+constexpr int kUpThreads = 8;
+constexpr size_t kUpMin = 24 << 20;
+struct UploadSlots {
+  std::mutex mu;
+  bool made = false, failed = false;
+  void * pinned[kUpThreads][2] = {};
+  cudaEvent_t sent[kUpThreads][2] = {};
+};
+std::mutex g_up_mu;
+std::map<int, UploadSlots *> g_up;
+
+// All of a device's slots, or none.
+bool make_slots(UploadSlots & u) {
+  if (u.made || u.failed) return u.made;
+  void * block = nullptr;
+  u.failed = true;
+  if (cudaHostAlloc(&block, kUpThreads * 2 * kUpPiece, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (int t = 0; t < kUpThreads; ++t)
+    for (int q = 0; q < 2; ++q) {
+      u.pinned[t][q] = static_cast<char *>(block) + (2 * t + q) * kUpPiece;
+      if (cudaEventCreateWithFlags(&u.sent[t][q], cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeHost(block);
+        return false;
+      }
+    }
+  u.failed = false;
+  return u.made = true;
+}
+}  // namespace
+
+int upload(void * dst, const void * src, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return GOOSEBERRY_SUCCESS;
+  const unsigned cores = std::thread::hardware_concurrency();
+  bool staged = bytes >= kUpMin && cores >= 4;
+  if (staged) {  // pinned and managed memory has a faster way
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
+    else staged = at.type == cudaMemoryTypeUnregistered;
+  }
+  int dev = 0;
+  UploadSlots * u = nullptr;
+  if (staged) {
+    GB_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_up_mu);
+    UploadSlots *& p = g_up[dev];
+    if (!p) p = new UploadSlots();
+    u = p;
+  }
+  std::unique_lock<std::mutex> mine;
+  if (u) mine = std::unique_lock<std::mutex>(u->mu, std::try_to_lock);
+  if (!u || !mine.owns_lock() || !make_slots(*u)) {
+    GB_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+    return GOOSEBERRY_SUCCESS;
+  }
+  const size_t pieces = (bytes + kUpPiece - 1) / kUpPiece;
+  std::atomic<size_t> next{0};
+  std::atomic<int> err{cudaSuccess};
+  const auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(dev);
+    for (int q = 0; e == cudaSuccess && err.load() == cudaSuccess; q ^= 1) {
+      const size_t k = next.fetch_add(1);
+      if (k >= pieces) break;
+      const size_t at = k * kUpPiece, len = std::min(kUpPiece, bytes - at);
+      e = cudaEventSynchronize(u->sent[t][q]);  // the slot's last piece has left
+      if (e != cudaSuccess) break;
+      std::memcpy(u->pinned[t][q], static_cast<const char *>(src) + at, len);
+      e = cudaMemcpyAsync(static_cast<char *>(dst) + at, u->pinned[t][q], len,
+          cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess) e = cudaEventRecord(u->sent[t][q], s);
+    }
+    if (e != cudaSuccess) err.store(e);
+  };
+  std::vector<std::thread> helpers;
+  const int threads = static_cast<int>(std::min<size_t>(std::min<size_t>(kUpThreads, cores / 2),
+      pieces));
+  try {
+    helpers.reserve(threads);
+    for (int t = 1; t < threads; ++t) helpers.emplace_back(work, t);
+  } catch (...) {
+    // fewer helpers: the pieces are dealt out as threads ask for them
+  }
+  work(0);
+  for (auto & h : helpers) h.join();
+  GB_CUDA_TRY(static_cast<cudaError_t>(err.load()));
+  return GOOSEBERRY_SUCCESS;
 }
 
 }  // namespace gb

@@ -859,9 +859,10 @@ namespace {
 template <typename T>
 int alloc_copy(void ** dst, const T * src, size_t n, bool device_src, cudaStream_t s) {
   GB_TRY(dev_alloc(dst, std::max<size_t>(n, 1) * sizeof(T)));
-  if (n)
-    GB_CUDA_TRY(cudaMemcpyAsync(*dst, src, n * sizeof(T),
-        device_src ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
+  if (n && device_src)
+    GB_CUDA_TRY(cudaMemcpyAsync(*dst, src, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
+  else if (n)
+    GB_TRY(gb::upload(*dst, src, n * sizeof(T), s));
   return GOOSEBERRY_SUCCESS;
 }
 
