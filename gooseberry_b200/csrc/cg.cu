@@ -1504,6 +1504,25 @@ __global__ void __launch_bounds__(kVecBlock) cg_add_kernel(size_t n, const doubl
     x[i] += d[i];
 }
 
+}  // namespace
+
+int launch_true_residual(uint32_t n, const uint32_t * rowptr, const uint32_t * rowind,
+    const double * val, const double * b, const double * x, double * r, double * partial,
+    unsigned grid, double * rr, unsigned * ticket, cudaStream_t stream) {
+  cg_true_residual_kernel<<<grid, kVecBlock, 0, stream>>>(n, rowptr, rowind, val, b, x, r, partial,
+      rr, ticket);
+  GB_CUDA_TRY(cudaGetLastError());
+  return GOOSEBERRY_SUCCESS;
+}
+
+int launch_add_to(size_t n, const double * d, double * x, unsigned grid, cudaStream_t stream) {
+  cg_add_kernel<<<grid, kVecBlock, 0, stream>>>(n, d, x);
+  GB_CUDA_TRY(cudaGetLastError());
+  return GOOSEBERRY_SUCCESS;
+}
+
+namespace {
+
 // A solve on the chip.  *done = false: a wait inside it was given up (some
 // other program holds SMs), and the graph path has to run the solve.
 //
@@ -1546,16 +1565,14 @@ int solve_resident(gb_cg * s, const double * b, double * x, double tol, int tol_
         GB_CUDA_TRY(cudaMemcpyAsync(refine ? s->xsum : x, s->x, s->n * sizeof(double),
             cudaMemcpyDeviceToDevice, stream));
       } else {
-        cg_add_kernel<<<g, kVecBlock, 0, stream>>>(s->n, s->x, s->xsum);
+        GB_TRY(launch_add_to(s->n, s->x, s->xsum, g, stream));
         ++launches;
       }
       iters += r.iter;
       rnorm = std::sqrt(r.rr);
       if (!refine || out.cancelled_waiting || status == GB_CG_NONFINITE || bnorm == 0.0) break;
-      cg_true_residual_kernel<<<g, kVecBlock, 0, stream>>>(static_cast<uint32_t>(s->n),
-          s->a->rowptr, s->a->rowind, s->a->val64, b, s->xsum, s->r, s->partial_a, s->rr_true_d,
-          s->ticket);
-      GB_CUDA_TRY(cudaGetLastError());
+      GB_TRY(launch_true_residual(static_cast<uint32_t>(s->n), s->a->rowptr, s->a->rowind,
+          s->a->val64, b, s->xsum, s->r, s->partial_a, g, s->rr_true_d, s->ticket, stream));
       GB_CUDA_TRY(cudaStreamSynchronize(stream));
       ++rounds;
       ++launches;

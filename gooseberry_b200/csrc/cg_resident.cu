@@ -79,7 +79,6 @@ constexpr int kResThreadsWide = 384, kResRowsWide = 19;
 // Up to here one CTA, which needs no exchange (variable coefficients, 1,600
 // rows: 2.68 us an iteration, 3.36 over four CTAs; 2,304 rows: 3.41 and 3.39).
 constexpr uint32_t kResOneCta = 2048;
-constexpr int kResMaxCtas = 160;          // tagged partials polled, 5 a lane
 constexpr unsigned long long kResWaitNs = 2000000000ull;
 
 // How a CTA finds its matrix rows.
@@ -91,11 +90,6 @@ enum ResSource {
   RES_GLOBAL_F32 = 4,  // pattern byte; rows of 8 exact floats in global memory
   RES_CODES = 5,   // pattern byte; rows of 8 value codes in global memory
   RES_CSR = 6      // the plain CSR arrays
-};
-
-// What has a place in shared memory besides p, Ap, the tables and the row bytes.
-struct ResPlaces {
-  int x, halo;  // x (else in L2); the neighbours' r as fetched (else not fetched ahead)
 };
 
 // Shared-memory regions, the same on host and device.
@@ -122,36 +116,6 @@ struct ResLayout {
     codes = o;
     total = (o + r + 15) / 16 * 16;
   }
-};
-
-struct ResArgs {
-  uint32_t n, rows, halo, ctas;
-  int tol_relative;
-  ResPlaces at;
-  const uint8_t * row_code;       // class or pattern of each row
-  const ResRowClass * classes;    // RES_CLASS
-  const int32_t * pat_off;        // the other pattern sources
-  uint32_t ncode;                 // classes or patterns
-  const void * vals;              // rows of values or codes
-  int val_width;                  // elements per row of `vals`
-  const double * table;           // RES_CODES
-  uint32_t ntable;
-  const uint32_t * rowptr;        // RES_CSR
-  const uint32_t * rowind;
-  const double * val64;
-  const double * b;
-  double * x;
-  ulonglong2 * r_edge;            // [n] tagged r; only rows near a block edge are used
-  unsigned long long * words;     // [2][16]: the fixed-point sums (3 of 16 used)
-  ulonglong2 * box;               // [2][ctas] tagged partials
-  int * abort_flag;
-  const int * cancel;
-  ResResult * out;                // host-mapped
-  double * hist;
-  unsigned long long hist_len, niter;
-  uint32_t epoch0;
-  double tol;
-  int timed;                      // report the phases' times
 };
 
 __host__ __device__ constexpr size_t res_val_bytes(int src, int stage) {
@@ -501,12 +465,21 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     for (uint32_t i = tid; i < nloc; i += T) codes[i] = a.row_code[lo + i];
     if constexpr (SRC == RES_SMEM_F64 || SRC == RES_SMEM_F32) {
       using V = typename std::conditional<SRC == RES_SMEM_F64, double, float>::type;
-      const V * g = reinterpret_cast<const V *>(a.vals) + static_cast<size_t>(a.val_width) * lo;
       V * s = reinterpret_cast<V *>(smem + L.vals);
-      const uint32_t m = nloc * a.val_width;
-      for (uint32_t i = tid; i < m; i += T) {
-        const uint32_t row = i / a.val_width, j = i - row * a.val_width;
-        if (j < STAGE) s[j * a.rows + row] = g[i];
+      if (a.vals) {  // rows of val_width values
+        const V * g = reinterpret_cast<const V *>(a.vals) + static_cast<size_t>(a.val_width) * lo;
+        const uint32_t m = nloc * a.val_width;
+        for (uint32_t i = tid; i < m; i += T) {
+          const uint32_t row = i / a.val_width, j = i - row * a.val_width;
+          if (j < STAGE) s[j * a.rows + row] = g[i];
+        }
+      } else {  // the CSR array
+        for (uint32_t i = tid; i < nloc; i += T) {
+          const uint32_t b = a.rowptr[lo + i], e = a.rowptr[lo + i + 1];
+#pragma unroll
+          for (int j = 0; j < STAGE; ++j)
+            s[j * a.rows + i] = b + j < e ? static_cast<V>(a.val64[b + j]) : V(0);
+        }
       }
     }
   }
@@ -834,6 +807,16 @@ bool resident_acquire(int device, unsigned ctas, unsigned capacity, const int * 
   return true;
 }
 
+bool resident_try_acquire(int device, unsigned ctas, unsigned capacity) {
+  ResGate & g = gate();
+  std::lock_guard<std::mutex> lk(g.mu);
+  if (g.next[device] != g.serving[device] ||
+      g.used[device] + std::min(ctas, capacity) > capacity)
+    return false;
+  g.used[device] += std::min(ctas, capacity);
+  return true;
+}
+
 void resident_release(int device, unsigned ctas, unsigned capacity) {
   ResGate & g = gate();
   std::lock_guard<std::mutex> lk(g.mu);
@@ -866,6 +849,51 @@ void resident_destroy(ResidentCg * s) {
   pinned_slot_free(s->out_h);
   free_row_classes(s->classes);
   delete s;
+}
+
+int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,
+    ResShape * out) {
+  *out = ResShape{};
+  int dev = 0, max_smem = 0;
+  GB_CUDA_TRY(cudaGetDevice(&dev));
+  GB_CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (n == 0 || max_row < 1 || max_row > 7 || npat == 0 || npat > 256) return GOOSEBERRY_SUCCESS;
+  const uint32_t cap = static_cast<uint32_t>(std::min(sms, kResMaxCtas));
+  const int stage = max_row <= 5 ? 5 : 7;
+  const size_t room = static_cast<size_t>(max_smem) - 1024;
+  for (uint32_t rows = want; rows >= 512; rows /= 2) {
+    const uint32_t parts = (n + rows - 1) / rows;  // equal parts of at most `rows`
+    const uint32_t r = ((n + parts - 1) / parts + 1) / 2 * 2, ctas = (n + r - 1) / r;
+    if (ctas > cap || r > kResThreads * kResRows) break;
+    const uint32_t halo = ctas > 1 ? std::min(half, n) : 0;
+    const auto need = [&](ResPlaces at) {
+      return ResLayout(r, halo, kResThreads, at, res_val_bytes(RES_SMEM_F64, stage),
+          res_table_bytes(RES_SMEM_F64, npat, 0)).total;
+    };
+    if (need(ResPlaces{1, 0}) > room) continue;
+    out->args.n = n;
+    out->args.rows = r;
+    out->args.halo = halo;
+    out->args.ctas = ctas;
+    out->args.ncode = npat;
+    out->args.at = ResPlaces{1, ctas > 1 && need(ResPlaces{1, 1}) <= room ? 1 : 0};
+    out->smem = need(out->args.at);
+    out->threads = kResThreads;
+    const int k = static_cast<int>((r + kResThreads - 1) / kResThreads);
+    const ResKernel fn = stage == 5 ? res_kernel_s<5>(RES_SMEM_F64, kResThreads, k)
+                                    : res_kernel_s<7>(RES_SMEM_F64, kResThreads, k);
+    out->fn = reinterpret_cast<const void *>(fn);
+    GB_TRY(raise_smem_limit(out->fn, out->smem));
+    return GOOSEBERRY_SUCCESS;
+  }
+  return GOOSEBERRY_SUCCESS;
+}
+
+int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream) {
+  void * kargs[] = {&args};
+  GB_CUDA_TRY(cudaLaunchCooperativeKernel(sh.fn, dim3(args.ctas), dim3(sh.threads), kargs, sh.smem,
+      stream));
+  return GOOSEBERRY_SUCCESS;
 }
 
 bool resident_size_ok(const gb_csr & a) {

@@ -52,6 +52,65 @@ struct ResResult {
   unsigned long long ns_a, ns_b;  // time in the two phases (a timed solve)
 };
 
+// ---- the solve kernel's arguments ------------------------------------------------
+// What has a place in shared memory besides p, Ap, the tables and the row bytes.
+struct ResPlaces {
+  int x, halo;  // x (else in L2); the neighbours' r as fetched (else not fetched ahead)
+};
+
+struct ResArgs {
+  uint32_t n, rows, halo, ctas;
+  int tol_relative;
+  ResPlaces at;
+  const uint8_t * row_code;       // class or pattern of each row
+  const ResRowClass * classes;    // RES_CLASS
+  const int32_t * pat_off;        // the other pattern sources
+  uint32_t ncode;                 // classes or patterns
+  const void * vals;              // rows of values or codes
+  int val_width;                  // elements per row of `vals`
+  const double * table;           // RES_CODES
+  uint32_t ntable;
+  const uint32_t * rowptr;        // RES_CSR
+  const uint32_t * rowind;
+  const double * val64;
+  const double * b;
+  double * x;
+  ulonglong2 * r_edge;            // [n] tagged r; only rows near a block edge are used
+  unsigned long long * words;     // [2][16]: the fixed-point sums (3 of 16 used)
+  ulonglong2 * box;               // [2][ctas] tagged partials
+  int * abort_flag;
+  const int * cancel;
+  ResResult * out;                // host-mapped
+  double * hist;
+  unsigned long long hist_len, niter;
+  uint32_t epoch0;
+  double tol;
+  int timed;                      // report the phases' times
+};
+
+// One solve's grid and kernel, from its size alone: matrix values in shared
+// memory, read from the CSR arrays (args.vals stays null).  fn is null when the
+// system does not fit.  `want`: rows a CTA should own.
+struct ResShape {
+  ResArgs args{};
+  const void * fn = nullptr;
+  size_t smem = 0;
+  int threads = 0;
+};
+int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,
+    ResShape * out);
+// Enqueue a solve.  The caller holds the grid's SMs (resident_acquire) until it
+// has ended, and has cleared words, box, abort flag and r_edge.
+int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream);
+constexpr int kResMaxCtas = 160;  // tagged partials polled, 5 a lane
+
+// r = b - A x and r.r into *rr (may be host-mapped), with `grid` partials and a
+// ticket that is 0 before and after; x += d (cg.cu).
+int launch_true_residual(uint32_t n, const uint32_t * rowptr, const uint32_t * rowind,
+    const double * val, const double * b, const double * x, double * r, double * partial,
+    unsigned grid, double * rr, unsigned * ticket, cudaStream_t stream);
+int launch_add_to(size_t n, const double * d, double * x, unsigned grid, cudaStream_t stream);
+
 struct ResOutcome {
   ResResult result{};
   bool cancelled_waiting = false;  // cancelled before it got its SMs
@@ -87,6 +146,8 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
 // SMs of a device shared by the grids whose CTAs wait for one another; false
 // if `cancel` (host, may be null) was set before the SMs were free.
 bool resident_acquire(int device, unsigned ctas, unsigned capacity, const int * cancel);
+// The same without waiting: false if the SMs are not free, or others wait.
+bool resident_try_acquire(int device, unsigned ctas, unsigned capacity);
 void resident_release(int device, unsigned ctas, unsigned capacity);
 
 }  // namespace gb

@@ -1,5 +1,7 @@
 // serve.cu -- batched CG serving: many uneven solves resident at once,
-// continuous batching, admission by device-memory footprint.
+// continuous batching, admission by device-memory footprint.  Requests whose
+// systems fit the SMs run there from start to end, side by side (see "solves
+// on the chip" below); the batch described next serves the others.
 //
 // Reference: one cgd call (src/cgd.c:40-129) runs at a time from the CLI
 // (src/gooseberry_bin.c:2078-2091).  Here every resident solve owns a slot:
@@ -52,6 +54,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cg_resident.h"
 #include "gb_internal.h"
 #include "spmv_tiles.cuh"
 #include "cg_common.cuh"
@@ -84,6 +87,44 @@ constexpr uint32_t kTileRows = GB_SRV_TILE_ROWS;
 constexpr uint32_t kMaxRowNnz = 255;      // longer rows belong to the single-solve CG
 constexpr double kSrvDelta = 0.1;         // reliable update trigger (see cg_mixed.cu)
 constexpr size_t kMaxTiles = 1u << 20;
+
+// ---- solves on the chip ------------------------------------------------------------
+//
+// A request whose matrix is a pattern matrix (rows of at most 7 entries, at
+// most 256 lists of column offsets) and whose rows fit the SMs' shared memory
+// is run from start to end by one launch of the on-chip solver
+// (cg_resident.cu) on as many SMs as it needs, beside those of other requests;
+// steps start queued solves as SMs come free and collect finished ones.  The
+// batch below serves the rest.
+//
+// The batch streams every vector of every solve through L2 or HBM each
+// iteration; on the chip only the edge values and two sums cross L2.  Measured
+// (ms, all requests submitted and drained, batch -> here): 48 requests of 1k to
+// 262k rows 269 -> 92; 8 of them 204 -> 47; 20 of 1k to 65k rows 73 -> 20; 40 of
+// 1k to 16k rows, FP64, 30 -> 23.
+//
+// Rows a CTA takes: more of them solve one request slower but leave SMs to
+// others.  2,048 up to 65,536 rows, past that 3,072 (the four cases above at
+// 2,048 throughout: 108, 47, 20, 23; at 3,072: 92, 48, 28, 27; at 1,024 large
+// systems do not fit).
+constexpr uint32_t srv_rows_per_cta(uint32_t n) { return n <= 65536 ? 2048 : 3072; }
+constexpr unsigned kSrvResidualGrid = 64;  // CTAs of the true-residual kernel
+constexpr uint32_t kSrvPatMax = 256;
+// Device control block of a slot: fixed-point words, tagged partials, abort
+// flag and ticket, residual partials.
+constexpr size_t kCtlBox = 256;
+constexpr size_t kCtlFlag = kCtlBox + 2 * kResMaxCtas * 16;
+constexpr size_t kCtlPart = kCtlFlag + 64;
+constexpr size_t kCtlBytes = kCtlPart + kSrvResidualGrid * 8;
+// Pinned, mapped block of a slot: the kernel's result, r.r of b - A x, the
+// cancel flag.
+struct SrvPinned {
+  ResResult res;
+  double rr_true;
+  int cancel;
+};
+constexpr size_t kPinnedStride = 256;
+static_assert(sizeof(SrvPinned) <= kPinnedStride, "a slot's pinned block");
 
 // What a launch does for a slot.  A: kWorkCg, kWorkInit or kWorkIdle;
 // B: kWorkUpdate, kWorkReliable or kWorkIdle.
@@ -626,6 +667,10 @@ struct Request {
   double t_submit = 0.0;
   size_t bytes = 0;
   std::vector<SrvTile> tiles;  // slot-relative (slot field filled at admission)
+  ResShape shape;              // a solve on the chip when shape.fn is set
+  uint8_t * codes = nullptr;   // its rows' patterns and their offset lists, staged
+  int32_t * pats = nullptr;    // like the arrays above
+  uint32_t npat = 0;
 };
 
 struct SlotHost {
@@ -637,14 +682,29 @@ struct SlotHost {
   double * x_out = nullptr;
   double t_submit = 0.0, t_admit = 0.0;
   std::vector<SrvTile> tiles;
+  // a solve on the chip
+  enum { kBatch, kWaiting, kRunning, kFinished } chip = kBatch;
+  ResShape shape;
+  SrvSlot dev{};                 // its device arrays (and the batch's, should it fall back)
+  double * d = nullptr;          // refinement's correction (mixed)
+  ulonglong2 * r_edge = nullptr;
+  uint8_t * codes = nullptr;
+  int32_t * pats = nullptr;
+  uint32_t npat = 0, nnz = 0;
+  int stream = -1;
+  cudaEvent_t copied = nullptr;  // set at admission, waited for by the first launch
+  double tol = 0.0, bnorm = 0.0, rnorm = 0.0;
+  size_t iters = 0, rounds = 0;
+  int status = GB_CG_MAXITER;
 };
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-// Host bytes of a queued request's arrays (rowptr, rowind, values, b).
+// Host bytes of a queued request's arrays (rowptr, rowind, values, b, row
+// patterns).
 size_t request_host_bytes(uint32_t n, uint32_t nnz) {
   return align256(4ull * (n + 1)) + align256(4ull * nnz) + align256(8ull * nnz) +
-         align256(8ull * n);
+         align256(8ull * n) + align256(n) + kSrvPatMax * kPatMax * 4;
 }
 
 }  // namespace
@@ -683,6 +743,14 @@ struct gb_server {
   cudaEvent_t step_done = nullptr;
   bool inflight = false;
   gb_server_stats_t stats{};
+  // solves on the chip
+  int device = 0;
+  unsigned char * d_ctl = nullptr;      // [max_slots] control blocks
+  unsigned char * h_pin = nullptr;      // [max_slots] pinned blocks
+  unsigned char * d_pin = nullptr;      // their device address
+  std::vector<cudaStream_t> streams;    // made as they are needed
+  std::vector<int> free_streams;
+  std::vector<cudaEvent_t> begin, end;  // per slot
 };
 
 namespace gb {
@@ -700,6 +768,16 @@ SrvDev dev_view(gb_server & s) {
   d.pa = s.d_part;
   d.pb = s.d_part + kMaxTiles;
   return d;
+}
+
+SrvPinned * pinned(gb_server & s, uint32_t k) {
+  return reinterpret_cast<SrvPinned *>(s.h_pin + k * kPinnedStride);
+}
+SrvPinned * pinned_dev(gb_server & s, uint32_t k) {
+  return reinterpret_cast<SrvPinned *>(s.d_pin + k * kPinnedStride);
+}
+unsigned chip_capacity(const gb_server & s) {
+  return static_cast<unsigned>(std::min(s.sm_count, kResMaxCtas));
 }
 
 int capture_graph(gb_server & s) {
@@ -731,6 +809,22 @@ int capture_graph(gb_server & s) {
 
 void destroy_server(gb_server * s) {
   if (!s) return;
+  for (uint32_t k = 0; k < s->slots.size(); ++k)  // running solves stop at their next check
+    if (s->slots[k].chip == SlotHost::kRunning && s->h_pin)
+      __atomic_store_n(&pinned(*s, k)->cancel, 1, __ATOMIC_RELEASE);
+  for (auto & st : s->streams) cudaStreamSynchronize(st);
+  for (auto & h : s->slots) {
+    if (h.chip == SlotHost::kRunning)
+      resident_release(s->device, h.shape.args.ctas, chip_capacity(*s));
+    if (h.copied) cudaEventDestroy(h.copied);
+  }
+  for (auto & st : s->streams) cudaStreamDestroy(st);
+  for (auto & e : s->begin)
+    if (e) cudaEventDestroy(e);
+  for (auto & e : s->end)
+    if (e) cudaEventDestroy(e);
+  cudaFree(s->d_ctl);
+  if (s->h_pin) cudaFreeHost(s->h_pin);
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->graph) cudaGraphExecDestroy(s->graph);
   if (s->step_done) cudaEventDestroy(s->step_done);
@@ -796,6 +890,14 @@ int create_server(const gb_server_config_t & cfg, gb_server * s) {
     }
   }
   *s->h_ntiles = 0;
+  GB_CUDA_TRY(cudaGetDevice(&s->device));
+  GB_CUDA_TRY(cudaMalloc(&s->d_ctl, cfg.max_slots * kCtlBytes));
+  GB_CUDA_TRY(cudaHostAlloc(&s->h_pin, cfg.max_slots * kPinnedStride,
+      cudaHostAllocMapped | cudaHostAllocPortable));
+  std::memset(s->h_pin, 0, cfg.max_slots * kPinnedStride);
+  GB_CUDA_TRY(cudaHostGetDevicePointer(&s->d_pin, s->h_pin, 0));
+  s->begin.assign(cfg.max_slots, nullptr);
+  s->end.assign(cfg.max_slots, nullptr);
   GB_CUDA_TRY(cudaMalloc(&s->d_part, 2 * kMaxTiles * sizeof(double2)));
   s->slots.resize(cfg.max_slots);
   GB_CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
@@ -815,6 +917,51 @@ size_t footprint(bool mixed, uint32_t n, uint32_t nnz) {
 }
 
 int tile_rows_for(gb_server & s, const Request & q, uint32_t maxrow, uint32_t * out);
+
+// The request's row patterns (a byte a row, lists of offsets from the
+// diagonal), its half bandwidth and, when it can be solved on the chip, the
+// shape of that solve.  The rows are checked already.
+int plan_on_chip(gb_server & s, Request & q, uint32_t maxrow) {
+  q.npat = 0;
+  if (maxrow < 1 || maxrow > 7) return GOOSEBERRY_SUCCESS;
+  uint32_t half = 0;
+  uint32_t last = 0;
+  for (uint32_t r = 0; r < q.n; ++r) {
+    const uint32_t b = q.rowptr[r], l = q.rowptr[r + 1] - b;
+    const auto is = [&](uint32_t p) {
+      const int32_t * o = q.pats + p * kPatMax;
+      if (static_cast<uint32_t>(o[kPatMax - 1]) != l) return false;
+      for (uint32_t j = 0; j < l; ++j)
+        if (q.rowind[b + j] - r != static_cast<uint32_t>(o[j])) return false;
+      return true;
+    };
+    uint32_t p = last;  // mostly the row before has it
+    if (p >= q.npat || !is(p)) {
+      for (p = 0; p < q.npat && !is(p); ++p) {
+      }
+      if (p == q.npat) {
+        if (q.npat == kSrvPatMax) return GOOSEBERRY_SUCCESS;
+        int32_t * o = q.pats + q.npat++ * kPatMax;
+        for (uint32_t j = 0; j + 1 < static_cast<uint32_t>(kPatMax); ++j) {
+          o[j] = j < l ? static_cast<int32_t>(q.rowind[b + j] - r) : 0;
+          half = std::max(half, static_cast<uint32_t>(std::abs(static_cast<int64_t>(o[j]))));
+        }
+        o[kPatMax - 1] = static_cast<int32_t>(l);
+      }
+    }
+    last = p;
+    q.codes[r] = static_cast<uint8_t>(p);
+  }
+  // room beside the request's own arrays (admit lays them out)
+  const size_t extra = align256(32ull * q.npat) + align256(q.n);
+  const size_t have = s.mixed ? align256(4ull * q.nnz) : 5 * align256(8ull * q.n);
+  const size_t need = s.mixed ? align256(8ull * q.n) + extra : align256(16ull * q.n) + extra;
+  if (need > have || 5 * align256((s.mixed ? 4ull : 8ull) * q.n) < 16ull * q.n)
+    return GOOSEBERRY_SUCCESS;
+  return resident_shape(q.n, half, static_cast<int>(maxrow), q.npat, s.sm_count,
+      srv_rows_per_cta(q.n),
+      &q.shape);
+}
 
 int submit(gb_server & s, uint64_t id, dim_t n, const ind_t * rowptr, const dim_t * rowind,
     const double * rowval, const double * b, double * x_out, double tol_rel, size_t niter) {
@@ -849,6 +996,10 @@ int submit(gb_server & s, uint64_t id, dim_t n, const ind_t * rowptr, const dim_
   q.val64 = reinterpret_cast<double *>(base + at);
   at += align256(8ull * nnz);
   q.b = reinterpret_cast<double *>(base + at);
+  at += align256(8ull * n);
+  q.codes = base + at;
+  at += align256(n);
+  q.pats = reinterpret_cast<int32_t *>(base + at);
   // checks run on the copy; a refused request hands its staging region back
   uint32_t maxrow = 0;
   const int rc = [&]() -> int {
@@ -878,7 +1029,7 @@ int submit(gb_server & s, uint64_t id, dim_t n, const ind_t * rowptr, const dim_
     GB_CHECK_INPUT(ntiles <= kMaxTiles, "request needs %zu tiles, more than %zu", ntiles,
         kMaxTiles);
     for (uint32_t r = 0; r < n; r += T) q.tiles.push_back(SrvTile{0, r, std::min(T, n - r), 0});
-    return GOOSEBERRY_SUCCESS;
+    return plan_on_chip(s, q, maxrow);
   }();
   if (rc != GOOSEBERRY_SUCCESS) {
     if (q.stage_len) s.stage_alloc.release(q.stage_off, q.stage_len);
@@ -943,7 +1094,30 @@ int admit(gb_server & s, Request & q, uint32_t k) {
     GB_CUDA_TRY(cudaMemcpyAsync(v64, q.val64, 8ull * q.nnz, cudaMemcpyHostToDevice, s.stream));
   }
   GB_CUDA_TRY(cudaMemcpyAsync(bb, q.b, 8ull * q.n, cudaMemcpyHostToDevice, s.stream));
-  if (s.mixed && q.nnz) GB_TRY(launch_round_f32(v64, v32, q.nnz, s.stream));
+  if (q.shape.fn) {
+    // its own arrays beside the request's: the edge values over y..Ap; the
+    // correction, patterns and row bytes over the float values (mixed), or
+    // behind the edge values
+    h.chip = SlotHost::kWaiting;
+    h.shape = q.shape;
+    h.npat = q.npat;
+    h.r_edge = static_cast<ulonglong2 *>(y);
+    char * more = s.mixed ? reinterpret_cast<char *>(v32)
+                          : static_cast<char *>(y) + align256(16ull * q.n);
+    if (s.mixed) {
+      h.d = reinterpret_cast<double *>(more);
+      more += align256(8ull * q.n);
+    }
+    h.pats = reinterpret_cast<int32_t *>(more);
+    h.codes = reinterpret_cast<uint8_t *>(more + align256(32ull * q.npat));
+    GB_CUDA_TRY(cudaMemcpyAsync(h.pats, q.pats, 32ull * q.npat, cudaMemcpyHostToDevice, s.stream));
+    GB_CUDA_TRY(cudaMemcpyAsync(h.codes, q.codes, q.n, cudaMemcpyHostToDevice, s.stream));
+    GB_CUDA_TRY(cudaEventCreateWithFlags(&h.copied, cudaEventDisableTiming));
+    GB_CUDA_TRY(cudaEventRecord(h.copied, s.stream));
+  } else if (s.mixed && q.nnz) {
+    GB_TRY(launch_round_f32(v64, v32, q.nnz, s.stream));
+  }
+  h.nnz = q.nnz;
   // the staging region goes back to the arena after the step's wait, when the
   // copies above are done; until every copy is queued the request keeps it
   if (q.stage_len) {
@@ -969,8 +1143,113 @@ int admit(gb_server & s, Request & q, uint32_t k) {
   S.a_work = kWorkInit;
   S.b_work = kWorkIdle;
   S.status = GB_CG_MAXITER;
+  h.dev = S;
+  if (h.chip != SlotHost::kBatch) return GOOSEBERRY_SUCCESS;  // the batch sees an empty slot
   s.h_slots[k] = S;
   s.dirty = true;
+  return GOOSEBERRY_SUCCESS;
+}
+
+// Enqueue a solve on the chip for slot k (the first, or with rounds > 0 the
+// correction A d = b - A x), and behind it, in mixed mode, the true residual.
+// The caller holds its SMs.
+int launch_on_chip(gb_server & s, uint32_t k) {
+  SlotHost & h = s.slots[k];
+  const SrvSlot & S = h.dev;
+  if (h.stream < 0) {
+    if (s.free_streams.empty()) {
+      cudaStream_t st = nullptr;
+      GB_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      s.streams.push_back(st);
+      s.free_streams.push_back(static_cast<int>(s.streams.size()) - 1);
+    }
+    h.stream = s.free_streams.back();
+    s.free_streams.pop_back();
+  }
+  cudaStream_t st = s.streams[h.stream];
+  if (!s.begin[k]) GB_CUDA_TRY(cudaEventCreate(&s.begin[k]));
+  if (!s.end[k]) GB_CUDA_TRY(cudaEventCreate(&s.end[k]));
+  unsigned char * ctl = s.d_ctl + k * kCtlBytes;
+  SrvPinned * pin = pinned(s, k);
+  std::memset(&pin->res, 0, sizeof(pin->res));
+  pin->rr_true = 0.0;
+  GB_CUDA_TRY(cudaStreamWaitEvent(st, h.copied, 0));
+  GB_CUDA_TRY(cudaMemsetAsync(ctl, 0, kCtlBytes, st));
+  GB_CUDA_TRY(cudaMemsetAsync(h.r_edge, 0, 16ull * h.n, st));
+  ResArgs a = h.shape.args;
+  a.tol_relative = h.rounds ? 0 : 1;
+  a.tol = h.rounds ? h.tol : S.tol_rel;
+  a.niter = S.niter - h.iters;
+  a.row_code = h.codes;
+  a.pat_off = h.pats;
+  a.rowptr = S.rowptr;
+  a.rowind = S.rowind;
+  a.val64 = S.val64;
+  a.b = h.rounds ? S.x1 : S.b;
+  a.x = h.rounds ? h.d : S.x0;
+  a.r_edge = h.r_edge;
+  a.words = reinterpret_cast<unsigned long long *>(ctl);
+  a.box = reinterpret_cast<ulonglong2 *>(ctl + kCtlBox);
+  a.abort_flag = reinterpret_cast<int *>(ctl + kCtlFlag);
+  a.cancel = &pinned_dev(s, k)->cancel;
+  a.out = &pinned_dev(s, k)->res;
+  a.epoch0 = 2;
+  GB_CUDA_TRY(cudaEventRecord(s.begin[k], st));
+  GB_TRY(resident_launch(h.shape, a, st));
+  if (s.mixed) {
+    if (h.rounds) GB_TRY(launch_add_to(h.n, h.d, S.x0, kSrvResidualGrid, st));
+    GB_TRY(launch_true_residual(h.n, S.rowptr, S.rowind, S.val64, S.b, S.x0, S.x1,
+        reinterpret_cast<double *>(ctl + kCtlPart), kSrvResidualGrid,
+        &pinned_dev(s, k)->rr_true, reinterpret_cast<unsigned *>(ctl + kCtlFlag + 16), st));
+  }
+  GB_CUDA_TRY(cudaEventRecord(s.end[k], st));
+  h.chip = SlotHost::kRunning;
+  return GOOSEBERRY_SUCCESS;
+}
+
+// Take slot k's ended solve: finished, to be corrected once more (mixed: the
+// recurrence met the tolerance before b - A x did), or back to the batch (a
+// wait inside it was given up).
+int collect_on_chip(gb_server & s, uint32_t k) {
+  SlotHost & h = s.slots[k];
+  const SrvPinned & pin = *pinned(s, k);
+  float ms = 0.f;
+  if (cudaEventElapsedTime(&ms, s.begin[k], s.end[k]) == cudaSuccess)  // its share of the device
+    s.stats.gpu_ms += ms * h.shape.args.ctas / std::max(1, s.sm_count);
+  resident_release(s.device, h.shape.args.ctas, chip_capacity(s));
+  s.free_streams.push_back(h.stream);
+  h.stream = -1;
+  if (pin.res.aborted) {
+    SrvSlot S = h.dev;
+    if (s.mixed && h.nnz)
+      GB_TRY(launch_round_f32(S.val64, const_cast<float *>(S.val32), h.nnz, s.stream));
+    cudaEventDestroy(h.copied);
+    h.copied = nullptr;
+    h.chip = SlotHost::kBatch;
+    s.h_slots[k] = S;
+    s.dirty = true;
+    return GOOSEBERRY_SUCCESS;
+  }
+  h.iters += pin.res.iter;
+  h.status = pin.res.status;
+  h.rnorm = std::sqrt(pin.res.rr);
+  if (h.rounds == 0) {
+    h.bnorm = pin.res.bnorm;
+    h.tol = h.dev.tol_rel * h.bnorm;
+  }
+  h.chip = SlotHost::kFinished;
+  if (s.mixed && h.bnorm != 0.0 && h.status != GB_CG_NONFINITE) {
+    ++h.rounds;
+    h.rnorm = std::sqrt(pin.rr_true);
+    if (!std::isfinite(h.rnorm)) {
+      h.status = GB_CG_NONFINITE;
+    } else if (h.status == GB_CG_CONVERGED && h.rnorm > h.tol) {
+      h.status = h.cancel ? GB_CG_CANCELLED : GB_CG_MAXITER;
+      if (h.iters < h.dev.niter && !h.cancel) h.chip = SlotHost::kWaiting;
+    } else if (h.status == GB_CG_MAXITER && h.rnorm <= h.tol) {
+      h.status = GB_CG_CONVERGED;
+    }
+  }
   return GOOSEBERRY_SUCCESS;
 }
 
@@ -1178,6 +1457,10 @@ int cancel(gb_server & s, uint64_t id) {
   for (auto & h : s.slots) {
     if (!h.used || h.id != id || h.cancel) continue;
     h.cancel = true;  // the step in flight may still run it; the next step retires it
+    if (h.chip == SlotHost::kRunning) {
+      for (uint32_t k = 0; k < s.cfg.max_slots; ++k)
+        if (&s.slots[k] == &h) __atomic_store_n(&pinned(s, k)->cancel, 1, __ATOMIC_RELEASE);
+    }
     return GOOSEBERRY_SUCCESS;
   }
   set_error("no queued or resident request with id %llu", static_cast<unsigned long long>(id));
@@ -1202,14 +1485,28 @@ int step(gb_server & s, size_t * active, size_t * queued) {
     for (const auto & r : s.stage_done) s.stage_alloc.release(r.first, r.second);
     s.stage_done.clear();
   }
+  // 0. collect the solves on the chip that have ended (a cancelled one stops
+  //    within 64 iterations)
+  bool moved = false;
+  for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
+    SlotHost & h = s.slots[k];
+    if (!h.used || h.chip != SlotHost::kRunning) continue;
+    cudaError_t e = h.cancel ? cudaEventSynchronize(s.end[k]) : cudaEventQuery(s.end[k]);
+    if (e == cudaErrorNotReady) continue;
+    GB_CUDA_TRY(e);
+    GB_TRY(collect_on_chip(s, k));
+    moved = true;
+  }
   // 1. retire finished (or cancelled) solves: copy x out, free memory and
   //    the slot
   bool any_done = false;
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
     const SrvSlot & S = s.h_slots[k];
-    if (!h.used || !S.done) continue;  // a solve that finished before its cancel keeps x
-    const double * x = (s.mixed && S.xpar) ? S.x1 : S.x0;
+    const bool on_chip = h.chip == SlotHost::kFinished && h.status != GB_CG_CANCELLED;
+    // a solve that finished before its cancel keeps x
+    if (!h.used || !(h.chip == SlotHost::kBatch ? S.done != 0 : on_chip)) continue;
+    const double * x = on_chip ? h.dev.x0 : (s.mixed && S.xpar) ? S.x1 : S.x0;
     GB_CUDA_TRY(cudaMemcpyAsync(h.x_out, x, 8ull * h.n, cudaMemcpyDeviceToHost, s.stream));
     any_done = true;
   }
@@ -1217,25 +1514,43 @@ int step(gb_server & s, size_t * active, size_t * queued) {
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
     SrvSlot & S = s.h_slots[k];
-    if (!h.used || !(S.done || h.cancel)) continue;
+    const bool batch = h.chip == SlotHost::kBatch;
+    if (!h.used || !((batch ? S.done != 0 : h.chip == SlotHost::kFinished) || h.cancel)) continue;
     gb_server_result_t res;
     res.id = h.id;
-    res.iterations = S.iter;
-    res.refinements = S.refinements;
-    res.rnorm = std::sqrt(S.rr_true);
-    res.bnorm = S.bnorm;
-    res.status = S.done ? S.status : GB_CG_CANCELLED;
+    if (batch) {
+      res.iterations = S.iter;
+      res.refinements = S.refinements;
+      res.rnorm = std::sqrt(S.rr_true);
+      res.bnorm = S.bnorm;
+      res.status = S.done ? S.status : GB_CG_CANCELLED;
+    } else {
+      res.iterations = h.iters;
+      res.refinements = h.rounds;
+      res.rnorm = h.rnorm;
+      res.bnorm = h.bnorm;
+      res.status = h.chip == SlotHost::kFinished ? h.status : GB_CG_CANCELLED;
+      if (h.copied) {
+        GB_CUDA_TRY(cudaEventSynchronize(h.copied));  // (cancelled before it was launched)
+        cudaEventDestroy(h.copied);
+      }
+      __atomic_store_n(&pinned(s, k)->cancel, 0, __ATOMIC_RELEASE);
+    }
     res.t_submit = h.t_submit;
     res.t_admit = h.t_admit;
     res.t_done = now_s(s);
     s.results.push_back(res);
     s.alloc.release(h.off, h.bytes);
+    if (batch) s.dirty = true;
     h = SlotHost();
     std::memset(&S, 0, sizeof(S));
-    s.dirty = true;
+    moved = true;
   }
   // 2. admit queued requests (FIFO; a request that does not fit yet lets a
   //    few later, smaller ones through rather than blocking them)
+  s.total_tiles = 0;  // of every resident request: one on the chip may fall back to the batch
+  for (const auto & h : s.slots)
+    if (h.used) s.total_tiles += h.tiles.size();
   size_t scanned = 0;
   for (auto it = s.queue.begin(); it != s.queue.end() && scanned < 16;) {
     uint32_t k = 0;
@@ -1249,6 +1564,32 @@ int step(gb_server & s, size_t * active, size_t * queued) {
     s.total_tiles += it->tiles.size();
     GB_TRY(admit(s, *it, k));
     it = s.queue.erase(it);
+    moved = true;
+  }
+  // 2b. start solves on the chip while SMs are free, the longest waiting first;
+  //     one that does not fit lets later, smaller ones through for 20 ms, then
+  //     SMs are kept for it
+  bool launched = false;
+  std::vector<uint32_t> wait;
+  for (uint32_t k = 0; k < s.cfg.max_slots; ++k)
+    if (s.slots[k].used && s.slots[k].chip == SlotHost::kWaiting && !s.slots[k].cancel)
+      wait.push_back(k);
+  std::sort(wait.begin(), wait.end(), [&](uint32_t p, uint32_t q) {
+    return s.slots[p].t_admit != s.slots[q].t_admit ? s.slots[p].t_admit < s.slots[q].t_admit
+                                                    : p < q;
+  });
+  for (uint32_t k : wait) {
+    const unsigned ctas = s.slots[k].shape.args.ctas;
+    if (!resident_try_acquire(s.device, ctas, chip_capacity(s))) {
+      if (now_s(s) - s.slots[k].t_admit > 0.02) break;
+      continue;
+    }
+    const int rc = launch_on_chip(s, k);
+    if (rc != GOOSEBERRY_SUCCESS) {
+      resident_release(s.device, ctas, chip_capacity(s));
+      return rc;
+    }
+    launched = true;
   }
   // 3. rebuild the tile list and upload the slot table
   size_t nact = 0;
@@ -1256,13 +1597,12 @@ int step(gb_server & s, size_t * active, size_t * queued) {
     size_t nt = 0;
     for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
       SlotHost & h = s.slots[k];
-      if (!h.used) continue;
+      if (!h.used || h.chip != SlotHost::kBatch) continue;
       s.h_slots[k].tile0 = static_cast<uint32_t>(nt);
       s.h_slots[k].ntiles = static_cast<uint32_t>(h.tiles.size());
       std::memcpy(s.h_tiles + nt, h.tiles.data(), h.tiles.size() * sizeof(SrvTile));
       nt += h.tiles.size();
     }
-    s.total_tiles = nt;
     *s.h_ntiles = static_cast<uint32_t>(nt);
     if (nt)
       GB_CUDA_TRY(cudaMemcpyAsync(s.d_tiles, s.h_tiles, nt * sizeof(SrvTile),
@@ -1273,9 +1613,33 @@ int step(gb_server & s, size_t * active, size_t * queued) {
         cudaMemcpyHostToDevice, s.stream));
     s.dirty = false;
   }
-  for (uint32_t k = 0; k < s.cfg.max_slots; ++k) nact += s.slots[k].used ? 1 : 0;
+  size_t nbatch = 0, running = 0;
+  for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
+    nact += s.slots[k].used ? 1 : 0;
+    nbatch += s.slots[k].used && s.slots[k].chip == SlotHost::kBatch ? 1 : 0;
+    running += s.slots[k].used && s.slots[k].chip == SlotHost::kRunning ? 1 : 0;
+  }
+  if (launched && !nbatch) s.stats.steps += 1;
+  // with nothing to do but wait for solves on the chip, wait for one (at most
+  // a millisecond, so that a caller's submissions and cancels get their turn)
+  if (running && !nbatch && !moved && !launched) {
+    const auto w0 = std::chrono::steady_clock::now();
+    bool ended = false;
+    while (!ended) {
+      for (uint32_t k = 0; k < s.cfg.max_slots && !ended; ++k)
+        if (s.slots[k].used && s.slots[k].chip == SlotHost::kRunning)
+          ended = cudaEventQuery(s.end[k]) != cudaErrorNotReady;
+      const double w = std::chrono::duration<double, std::milli>(
+          std::chrono::steady_clock::now() - w0).count();
+      if (ended || w > 1.0) {
+        waited += w;
+        s.stats.wait_ms += w;
+        break;
+      }
+    }
+  }
   // 4. run the step and bring the slot table back
-  if (nact) {
+  if (nbatch) {
     GB_CUDA_TRY(cudaEventRecord(s.step_start, s.stream));
     GB_CUDA_TRY(cudaGraphLaunch(s.graph, s.stream));
     GB_CUDA_TRY(cudaMemcpyAsync(s.h_slots, s.d_slots, s.cfg.max_slots * sizeof(SrvSlot),

@@ -380,7 +380,12 @@ GOOSEBERRY_API int gb_cg_row_bytes(const gb_cg_t * s, size_t * bytes);
 
 /*
  * Many independent CG solves of uneven sizes resident on one GPU at once.
- * Every gb_server_step runs `iters_per_step` CG iterations of EVERY resident
+ * Requests whose systems fit the SMs' shared memory (stencils: at most 7
+ * entries a row, at most 256 lists of column offsets) are each solved by one
+ * launch on as many SMs as they need, started by gb_server_step as SMs come
+ * free (in FP64 also under GB_CG_MIXED, which judges them on b - A x); the
+ * batch serves the others.
+ * Every gb_server_step runs `iters_per_step` CG iterations of EVERY batched
  * solve with one replay of a captured CUDA graph (the kernels walk a global
  * list of small row tiles covering all resident solves, so a 1k-row and a
  * 262k-row system advance together), retires the solves that finished
@@ -400,7 +405,8 @@ typedef struct gb_server_config {
   size_t pool_bytes;        /* device memory for resident solves             */
   uint32_t max_slots;       /* resident solves at most                       */
   int mode;                 /* GB_CG_MIXED or GB_CG_F64                      */
-  uint32_t iters_per_step;  /* CG iterations per gb_server_step (>= 1)       */
+  uint32_t iters_per_step;  /* CG iterations of the batch per gb_server_step
+                               (>= 1)                                        */
   uint32_t tile_rows;       /* rows per work tile (a power of two in
                                [256, 65536]), or 0: chosen per request by the
                                tile autotuner (gb_server_tuned_tile_rows)    */
@@ -430,7 +436,8 @@ GOOSEBERRY_API int gb_server_submit(gb_server_t * s, uint64_t id, dim_t n,
     double * x_out, double tol_rel, size_t niter);
 
 /* One scheduling step (see above).  Returns at once after queueing the
- * step's GPU work; *active / *queued (optional) receive the resident and
+ * step's GPU work; with nothing to queue while solves run on the chip, it
+ * waits for one of them to end, at most a millisecond.  *active / *queued (optional) receive the resident and
  * waiting request counts. */
 GOOSEBERRY_API int gb_server_step(gb_server_t * s, size_t * active, size_t * queued);
 
@@ -451,8 +458,9 @@ GOOSEBERRY_API double gb_server_clock(const gb_server_t * s);
 
 /* Where a server's time went. */
 typedef struct gb_server_stats {
-  size_t steps;             /* graph replays launched                        */
-  double gpu_ms;            /* their device time (CUDA events)               */
+  size_t steps;             /* steps that launched GPU work                  */
+  double gpu_ms;            /* its device time (CUDA events; a solve on the
+                               chip counts by its share of the SMs)          */
   double wait_ms;           /* host time in gb_server_step waiting for the
                                previous replay to finish                     */
   double host_ms;           /* the rest of gb_server_step: retiring, admitting,
