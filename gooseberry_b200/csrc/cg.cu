@@ -1515,6 +1515,13 @@ int launch_true_residual(uint32_t n, const uint32_t * rowptr, const uint32_t * r
   return GOOSEBERRY_SUCCESS;
 }
 
+int preload_true_residual() {
+  cudaFuncAttributes at;
+  GB_CUDA_TRY(cudaFuncGetAttributes(&at, cg_true_residual_kernel));
+  GB_CUDA_TRY(cudaFuncGetAttributes(&at, cg_add_kernel));
+  return GOOSEBERRY_SUCCESS;
+}
+
 int launch_add_to(size_t n, const double * d, double * x, unsigned grid, cudaStream_t stream) {
   cg_add_kernel<<<grid, kVecBlock, 0, stream>>>(n, d, x);
   GB_CUDA_TRY(cudaGetLastError());

@@ -889,6 +889,17 @@ int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sm
   return GOOSEBERRY_SUCCESS;
 }
 
+int resident_preload() {
+  cudaFuncAttributes at;
+  for (int k : {1, 4, kResRows}) {
+    GB_CUDA_TRY(cudaFuncGetAttributes(&at,
+        reinterpret_cast<const void *>(res_kernel_s<5>(RES_SMEM_F64, kResThreads, k))));
+    GB_CUDA_TRY(cudaFuncGetAttributes(&at,
+        reinterpret_cast<const void *>(res_kernel_s<7>(RES_SMEM_F64, kResThreads, k))));
+  }
+  return GOOSEBERRY_SUCCESS;
+}
+
 int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream) {
   void * kargs[] = {&args};
   GB_CUDA_TRY(cudaLaunchCooperativeKernel(sh.fn, dim3(args.ctas), dim3(sh.threads), kargs, sh.smem,

@@ -99,6 +99,10 @@ struct ResShape {
 };
 int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,
     ResShape * out);
+// Load every kernel that resident_shape may choose.  A kernel is otherwise
+// loaded at its first use, and what is launched after a load waits until the
+// kernels that run have ended: a request behind a long solve would wait for it.
+int resident_preload();
 // Enqueue a solve.  The caller holds the grid's SMs (resident_acquire) until it
 // has ended, and has cleared words, box, abort flag and r_edge.
 int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream);
@@ -110,6 +114,7 @@ int launch_true_residual(uint32_t n, const uint32_t * rowptr, const uint32_t * r
     const double * val, const double * b, const double * x, double * r, double * partial,
     unsigned grid, double * rr, unsigned * ticket, cudaStream_t stream);
 int launch_add_to(size_t n, const double * d, double * x, unsigned grid, cudaStream_t stream);
+int preload_true_residual();  // loads the two kernels above
 
 struct ResOutcome {
   ResResult result{};

@@ -193,6 +193,7 @@ int launch_spmm_fused(const gb_csr & a, uint32_t k, const T * vals, const T * b,
 int launch_max_index(const uint32_t * rowind, uint32_t nnz, unsigned int * d_out,
     cudaStream_t stream);
 int launch_round_f32(const double * in, float * out, size_t n, cudaStream_t stream);
+int preload_round_f32();  // loads its kernel
 
 int sm_count_of_current_device(int * out);
 // Whether `bytes` of working set fit in the current device's L2 (the CG

@@ -904,7 +904,9 @@ int create_server(const gb_server_config_t & cfg, gb_server * s) {
   GB_CUDA_TRY(cudaEventCreate(&s->step_start));
   GB_CUDA_TRY(cudaEventCreate(&s->step_done));
   GB_TRY(capture_graph(*s));
-  return GOOSEBERRY_SUCCESS;
+  GB_TRY(resident_preload());
+  GB_TRY(preload_true_residual());
+  return preload_round_f32();
 }
 
 size_t footprint(bool mixed, uint32_t n, uint32_t nnz) {

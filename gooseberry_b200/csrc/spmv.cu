@@ -637,6 +637,12 @@ int launch_round_f32(const double * in, float * out, size_t n, cudaStream_t stre
   return GOOSEBERRY_SUCCESS;
 }
 
+int preload_round_f32() {
+  cudaFuncAttributes at;
+  GB_CUDA_TRY(cudaFuncGetAttributes(&at, round_f32_kernel));
+  return GOOSEBERRY_SUCCESS;
+}
+
 // ---- autotuner --------------------------------------------------------------
 
 namespace {

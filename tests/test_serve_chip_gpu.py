@@ -4,6 +4,10 @@ wide) in one mix, both modes, the same bits alone and in the mix; a cancelled
 running solve; more requests than slots and SMs at once."""
 from __future__ import annotations
 
+import pathlib
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -83,14 +87,16 @@ def test_many_requests_and_a_running_one_cancelled():
     srv = gb.Server(pool_bytes=1 << 30, max_slots=16, mode=gb.CG_F64)
     A = W.diffusion_2d(300, 11)
     x = np.full(A.nrows, 3.0)
+    reqs = [(k, W.diffusion_2d(20 + 7 * k, 20 + k)) for k in range(40)]
+    for k, B in reqs[:10]:
+        srv.submit(k, B, W.rhs(B.nrows, k), tol=1e-8, niter=20_000)
+    srv.step()
+    # (r.r underflows to zero, which may end a solve early)
     srv.submit(1000, A, W.rhs(A.nrows, 1), tol=1e-300, niter=10 ** 7, x_out=x)
     srv.step()
-    reqs = [(k, W.diffusion_2d(20 + 7 * k, 20 + k)) for k in range(40)]
-    for k, B in reqs:
-        srv.submit(k, B, W.rhs(B.nrows, k), tol=1e-8, niter=20_000)
-    for _ in range(5):
-        srv.step()
     srv.cancel(1000)
+    for k, B in reqs[10:]:
+        srv.submit(k, B, W.rhs(B.nrows, k), tol=1e-8, niter=20_000)
     res = {r.id: r for r in srv.drain()}
     assert res[1000].status == "cancelled" and np.all(x == 3.0)
     for k, B in reqs:
@@ -98,6 +104,32 @@ def test_many_requests_and_a_running_one_cancelled():
         assert np.linalg.norm(W.rhs(B.nrows, k) - B.to_scipy() @ res[k].x) <= \
             2e-8 * np.linalg.norm(W.rhs(B.nrows, k))
     srv.close()
+
+
+BEHIND = """
+import sys
+import gooseberry_b200 as gb
+from gooseberry_b200 import workloads as W
+mode = int(sys.argv[1])
+srv = gb.Server(pool_bytes=1 << 29, max_slots=8, mode=mode)
+A = W.diffusion_2d(300, 11)
+reqs = [(k, W.diffusion_2d(w, k)) for k, w in enumerate((20, 40, 60, 100, 200))]
+srv.submit(1000, A, W.rhs(A.nrows, 1), tol=1e-300, niter=400_000)
+srv.step()
+for k, B in reqs:
+    srv.submit(k, B, W.rhs(B.nrows, k), tol=1e-8, niter=20_000)
+order = [r.id for r in srv.drain()]
+assert order[-1] == 1000 and sorted(order[:-1]) == [0, 1, 2, 3, 4], order
+srv.close()
+"""
+
+
+@pytest.mark.parametrize("mode", [gb.CG_F64, gb.CG_MIXED])
+def test_requests_behind_a_long_one(mode):
+    """In a new process, where no kernel is loaded yet: small requests (which
+    tune their tiles and take other kernels) end before a long one does."""
+    subprocess.run([sys.executable, "-c", BEHIND, str(mode)], check=True, timeout=300,
+                   cwd=pathlib.Path(__file__).parent.parent)
 
 
 def test_close_while_solves_run():
