@@ -1372,7 +1372,7 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
     // iterations wait for exchanges and shared memory, not for the bytes that
     // floats would save, and convergence is still judged on b - A x.
     if (a->sched64 != GB_SCHED_ROW || a->nnz == 0 || !resident_size_ok(*a))
-      return GOOSEBERRY_SUCCESS;
+      return mixed_past_chip(s->mixed);
     GB_TRY(dev_alloc(&s->x, std::max<size_t>(s->n, 2) * sizeof(double)));
     if (!plain_entries) {
       GB_TRY(build_row_codec(*a, &s->codec, nullptr));

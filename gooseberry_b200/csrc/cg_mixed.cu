@@ -35,6 +35,7 @@
 // solve stops at its iteration limit, and times the FP64 residual for the
 // profiler.
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 #include <vector>
 
@@ -361,6 +362,62 @@ __global__ void __launch_bounds__(kSpmvBlock, GB_MIX_PAT_MIN_BLOCKS) cg_a32_ell_
       r_cur = r_nx;
       p_cur = p_nx;
     }
+  }
+  __shared__ double red[32];
+  const double bs = block_sum(local, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
+}
+
+// A32 over symmetric diagonals (SymDiags): 16 bytes of matrix a row of a
+// 7-entry stencil instead of 33, no pattern, and every load of a warp a
+// contiguous run (the rows of 8 make each 16-byte load touch 32 rows: 8 L1
+// wavefronts).  All of a row's loads are independent of one another, so
+// nothing is staged a row ahead.  Same rows per thread, same order of products
+// (missing entries add 0 times a neighbour, or are left out past the matrix's
+// ends): the iterates are those of the other layouts.  Per iteration (A32 and
+// B32, rows of 8 -> here): 160^3 58.9 -> 55.5 us, 131^3 34.1 -> 33.2, 1500^2 32.3
+// -> 27.7.  It waits for its 21 loads a row rather than for bytes: a contiguous
+// block of rows per CTA, which would halve the L2 reads of r and p, measured
+// 54.7, 34.4 and 27.8, four to eight CTAs per SM 53 to 62 on the first.
+template <bool HINT, int ND>
+__global__ void __launch_bounds__(kSpmvBlock, GB_MIX_PAT_MIN_BLOCKS) cg_a32_sym_kernel(
+    uint32_t n, const float * __restrict__ u, uint4 off, const float * __restrict__ r,
+    const float * __restrict__ pold, float * __restrict__ pnew, float * __restrict__ ap,
+    double * __restrict__ partial, MixState * st, int par, const double * __restrict__ partial_b,
+    unsigned nb) {
+  pdl_wait_and_release();
+  if (mix_cta_done(st)) return;
+  float beta;
+  if (!mix_a_step(st, par, partial_b, nb, &beta)) return;
+  const auto pm = L2Pol<HINT>::stream();
+  const auto px = L2Pol<HINT>::keep();
+  const uint32_t d[4] = {0, off.y, off.z, off.w};
+  double local = 0.0;
+  const uint32_t step = gridDim.x * kSpmvBlock;
+  for (uint32_t i = blockIdx.x * kSpmvBlock + threadIdx.x; i < n; i += step) {
+    float lo[ND], lr[ND], lp[ND], up[ND], ur[ND], upo[ND];
+#pragma unroll
+    for (int k = 0; k < ND; ++k) {
+      const bool below = i >= d[k + 1], above = d[k + 1] < n - i;
+      const float * uk = u + static_cast<size_t>(k + 1) * n + i;
+      lo[k] = below ? ld_l1(uk - d[k + 1], pm) : 0.0f;
+      lr[k] = below ? ld_keep(r + i - d[k + 1], px) : 0.0f;
+      lp[k] = below ? ld_keep(pold + i - d[k + 1], px) : 0.0f;
+      up[k] = above ? ld_l1(uk, pm) : 0.0f;
+      ur[k] = above ? ld_keep(r + i + d[k + 1], px) : 0.0f;
+      upo[k] = above ? ld_keep(pold + i + d[k + 1], px) : 0.0f;
+    }
+    const float dv = ld_l1(u + i, pm), rc = ld_keep(r + i, px), pc = ld_keep(pold + i, px);
+    float sum = 0.0f;
+#pragma unroll
+    for (int k = ND - 1; k >= 0; --k) sum = add_rn(sum, mul_rn(lo[k], fmaf(beta, lp[k], lr[k])));
+    const float pn = fmaf(beta, pc, rc);
+    sum = add_rn(sum, mul_rn(dv, pn));
+#pragma unroll
+    for (int k = 0; k < ND; ++k) sum = add_rn(sum, mul_rn(up[k], fmaf(beta, upo[k], ur[k])));
+    ap[i] = sum;
+    pnew[i] = pn;
+    local += static_cast<double>(pn) * static_cast<double>(sum);
   }
   __shared__ double red[32];
   const double bs = block_sum(local, red);
@@ -784,6 +841,7 @@ struct MixedCg {
   float * p[2] = {nullptr, nullptr};
   float * ap = nullptr;
   float * v8 = nullptr;  // FP32 values in rows of 8 (pattern matrices, GB_MIX_ELL)
+  SymDiags sym;          // or, symmetric ones past the chip and L2, by diagonals
   double * partial_a = nullptr;
   double * partial_b = nullptr;
   double * partial_r = nullptr;
@@ -807,6 +865,20 @@ namespace {
 int launch_a32(MixedCg * m, cudaStream_t s, bool pdl, int k) {
   const float * pold = m->p[k & 1];
   float * pnew = m->p[(k + 1) & 1];
+  if (m->sym.u) {
+    const auto pick = [&](auto h) {
+      constexpr bool H = decltype(h)::value;
+      return m->sym.nd == 1 ? cg_a32_sym_kernel<H, 1>
+             : m->sym.nd == 2 ? cg_a32_sym_kernel<H, 2> : cg_a32_sym_kernel<H, 3>;
+    };
+    auto kern = m->l2_hint ? pick(std::true_type{}) : pick(std::false_type{});
+    GB_CUDA_TRY(launch_k(kern, m->grid_a, kSpmvBlock, 0, s, pdl, static_cast<uint32_t>(m->n),
+        static_cast<const float *>(m->sym.u),
+        make_uint4(0, m->sym.off[1], m->sym.off[2], m->sym.off[3]),
+        static_cast<const float *>(m->r), pold, pnew, m->ap, m->partial_a, m->st, k & 1,
+        static_cast<const double *>(m->partial_b), m->grid_b));
+    return GOOSEBERRY_SUCCESS;
+  }
   if (m->v8) {
     auto kern = m->stage == 5 ? (m->l2_hint ? cg_a32_ell_kernel<true, 5> : cg_a32_ell_kernel<false, 5>)
                               : (m->l2_hint ? cg_a32_ell_kernel<true, 7> : cg_a32_ell_kernel<false, 7>);
@@ -953,19 +1025,23 @@ void mixed_destroy(MixedCg * m) {
   dev_free(m->st);
   if (m->col16) dev_free(m->col16);
   if (m->v8) dev_free(m->v8);
+  if (m->sym.u) dev_free(m->sym.u);
   free_row_patterns(m->pat);
   pinned_slot_free(m->host_status);
   delete m;
 }
 
-// Stored bytes A32 streams per nonzero and per row: rows of 8 padded values
+// Stored bytes A32 streams per nonzero and per row: symmetric diagonals
+// (nothing per nonzero, no rowptr), rows of 8 padded values
 // and a pattern byte (ELL: nothing per nonzero, no rowptr), else rowptr plus a
 // pattern byte and a float per nonzero, 16-bit distances, or plain columns.
 size_t mixed_entry_bytes(const MixedCg * m) {
-  return m->v8 ? 0 : (m->pat.code8 ? 4 : (m->col16 ? 6 : 8));
+  return m->v8 || m->sym.u ? 0 : (m->pat.code8 ? 4 : (m->col16 ? 6 : 8));
 }
 
-size_t mixed_row_bytes(const MixedCg * m) { return m->v8 ? 33 : (m->pat.code8 ? 5 : 4); }
+size_t mixed_row_bytes(const MixedCg * m) {
+  return m->sym.u ? 4 * (m->sym.nd + 1) : m->v8 ? 33 : (m->pat.code8 ? 5 : 4);
+}
 
 int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out) {
   GB_CHECK_INPUT(a->val64 && a->val32,
@@ -1039,6 +1115,31 @@ int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out) {
   GB_TRY(capture(m, 0));
   GB_TRY(capture(m, 1));
   return GOOSEBERRY_SUCCESS;
+}
+
+int mixed_past_chip(MixedCg * m) {
+  // The diagonals win where the rows of 8 and their vectors, 57 bytes a row,
+  // no longer sit in L2. Per iteration, rows of 8 -> diagonals: 120^3 (98 MB)
+  // 26.2 -> 27.6 us and 1200^2 (82 MB) 20.7 -> 20.8; 131^3 (128 MB) 34.1 -> 33.2,
+  // 1500^2 (128 MB) 32.3 -> 27.7, 145^3 45.5 -> 42.3, 160^3 58.9 -> 55.5,
+  // 1900^2 49.5 -> 40.4. The line: 7/8 of L2 (116 MB).
+  bool l2 = true;
+  if (m->v8) GB_TRY(l2_fits((mixed_row_bytes(m) + 24ull) * m->n / 7 * 8, &l2));
+  if (l2) return GOOSEBERRY_SUCCESS;
+  if (build_sym_diags(*m->a, m->pat, m->a->val32, &m->sym, nullptr) != GOOSEBERRY_SUCCESS ||
+      !m->sym.u) {
+    cudaGetLastError();  // no memory for them, or not symmetric: the rows of 8 stay
+    return GOOSEBERRY_SUCCESS;
+  }
+  dev_free(m->v8);
+  m->v8 = nullptr;
+  for (auto & g : m->graph) {  // captured over the rows of 8
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+  GB_TRY(l2_fits(mixed_row_bytes(m) * (m->n + 1) + 24ull * m->n, &m->l2_hint));
+  GB_TRY(capture(m, 0));
+  return capture(m, 1);
 }
 
 namespace {

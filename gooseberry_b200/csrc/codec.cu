@@ -306,6 +306,53 @@ __global__ void codec_class_encode_kernel(const uint32_t * __restrict__ rowptr,
   }
 }
 
+// ---- symmetric diagonals -----------------------------------------------------------
+
+__global__ void codec_sym_fill_kernel(const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const float * __restrict__ val, uint32_t n, int nd,
+    uint4 off, float * __restrict__ u) {
+  const uint32_t o[4] = {off.x, off.y, off.z, off.w};
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const uint32_t e = __ldg(rowptr + i + 1);
+    for (uint32_t k = __ldg(rowptr + i); k < e; ++k) {
+      const uint32_t c = __ldg(rowind + k);
+      if (c < i) continue;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q <= nd && c - i == o[q]) v[q] = __ldg(val + k);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q <= nd) u[static_cast<size_t>(q) * n + i] = v[q];
+  }
+}
+
+// *bad = 1 where a row's entries below the diagonal (0 where missing) are not
+// those above it, bit for bit.
+__global__ void codec_sym_check_kernel(const uint32_t * __restrict__ rowptr,
+    const uint32_t * __restrict__ rowind, const float * __restrict__ val, uint32_t n, int nd,
+    uint4 off, const float * __restrict__ u, unsigned * bad) {
+  const uint32_t o[4] = {off.x, off.y, off.z, off.w};
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const uint32_t e = __ldg(rowptr + i + 1);
+    for (uint32_t k = __ldg(rowptr + i); k < e; ++k) {
+      const uint32_t c = __ldg(rowind + k);
+      if (c >= i) break;
+#pragma unroll
+      for (int q = 1; q < 4; ++q)
+        if (q <= nd && i - c == o[q]) v[q] = __ldg(val + k);
+    }
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (q <= nd) {
+        const float w = i >= o[q] ? u[static_cast<size_t>(q) * n + i - o[q]] : 0.0f;
+        if (value_bits(v[q]) != value_bits(w)) atomicExch(bad, 1u);
+      }
+  }
+}
+
 int grid_of(const gb_csr & a, size_t items) {
   const size_t want = (items + 255) / 256;
   return static_cast<int>(std::max<size_t>(1, std::min<size_t>(want,
@@ -508,6 +555,49 @@ int build_classes(const gb_csr & a, const T * val, RowClasses * out, cudaStream_
   return rc;
 }
 }  // namespace
+
+int build_sym_diags(const gb_csr & a, const RowPatterns & pat, const float * val, SymDiags * out,
+    cudaStream_t s) {
+  *out = SymDiags{};
+  if (!pat.code8 || !val || a.nrows != a.ncols) return GOOSEBERRY_SUCCESS;
+  std::vector<int32_t> off(static_cast<size_t>(pat.npat) * kPatMax);
+  GB_CUDA_TRY(cudaMemcpyAsync(off.data(), pat.off, off.size() * 4, cudaMemcpyDeviceToHost, s));
+  GB_CUDA_TRY(cudaStreamSynchronize(s));
+  std::vector<uint32_t> dist;
+  for (uint32_t p = 0; p < pat.npat; ++p) {
+    const int32_t * o = off.data() + p * kPatMax;
+    for (int j = 0; j < o[kPatMax - 1]; ++j) {
+      if (j && o[j] <= o[j - 1]) return GOOSEBERRY_SUCCESS;  // not in ascending order
+      const uint32_t d = static_cast<uint32_t>(o[j] < 0 ? -static_cast<int64_t>(o[j]) : o[j]);
+      if (d && std::find(dist.begin(), dist.end(), d) == dist.end()) dist.push_back(d);
+    }
+    if (dist.size() > 3) return GOOSEBERRY_SUCCESS;
+  }
+  if (dist.empty()) return GOOSEBERRY_SUCCESS;
+  std::sort(dist.begin(), dist.end());
+  out->nd = static_cast<int>(dist.size());
+  for (size_t q = 0; q < dist.size(); ++q) out->off[q + 1] = dist[q];
+  const uint4 o = make_uint4(0, out->off[1], out->off[2], out->off[3]);
+  unsigned * flag = nullptr;
+  unsigned bad = 1;
+  int rc = dev_alloc(&out->u, static_cast<size_t>(out->nd + 1) * a.nrows * sizeof(float));
+  if (rc == GOOSEBERRY_SUCCESS) rc = scratch_alloc(reinterpret_cast<void **>(&flag), 16, s);
+  if (rc == GOOSEBERRY_SUCCESS && cudaMemsetAsync(flag, 0, 16, s) != cudaSuccess)
+    rc = GOOSEBERRY_ERROR_UNKNOWN;
+  if (rc == GOOSEBERRY_SUCCESS) {
+    codec_sym_fill_kernel<<<grid_of(a, a.nrows), 256, 0, s>>>(a.rowptr, a.rowind, val, a.nrows,
+        out->nd, o, out->u);
+    codec_sym_check_kernel<<<grid_of(a, a.nrows), 256, 0, s>>>(a.rowptr, a.rowind, val, a.nrows,
+        out->nd, o, out->u, flag);
+    rc = read_flag(flag, &bad, s);
+  }
+  scratch_free(flag, s);
+  if (rc != GOOSEBERRY_SUCCESS || bad) {
+    if (out->u) dev_free(out->u);
+    *out = SymDiags{};
+  }
+  return rc;
+}
 
 int build_row_classes(const gb_csr & a, const double * val, RowClasses * out, cudaStream_t s) {
   return build_classes(a, val, out, s);

@@ -245,6 +245,21 @@ struct RowPatterns {
 int build_row_patterns(const gb_csr & a, RowPatterns * out, cudaStream_t s);
 void free_row_patterns(RowPatterns & p);
 
+// A symmetric pattern matrix by its diagonals: u[k n + i] = a(i, i + off[k]),
+// off[0] = 0 < off[1] < ... (0 where the entry is missing); the entry below the
+// diagonal is a(i, i - off[k]) = u[k n + i - off[k]].  Half the bytes of the
+// rows, and every load of a warp is one contiguous run.
+struct SymDiags {
+  float * u = nullptr;
+  int nd = 0;            // diagonals above the main one, 1 to 3
+  uint32_t off[4] = {0, 0, 0, 0};
+};
+// Built when the patterns' offsets, ascending in every row, are 0 and at most
+// three distances each way and a(i, j) = a(j, i) bit for bit; else `out` stays
+// empty.
+int build_sym_diags(const gb_csr & a, const RowPatterns & pat, const float * val, SymDiags * out,
+    cudaStream_t s);
+
 struct RowCodec {
   int16_t * col16 = nullptr;  // col - row
   uint8_t * code8 = nullptr;  // code of each value
@@ -267,6 +282,9 @@ int row_stage_for(const gb_csr & a);
 // Mixed-precision CG (cg_mixed.cu), owned by a gb_cg created with GB_CG_MIXED.
 struct MixedCg;
 int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out);
+// Lay a symmetric pattern matrix that exceeds L2 out by its diagonals
+// (SymDiags): for a solver whose solves do not run on the chip.
+int mixed_past_chip(MixedCg * m);
 size_t mixed_entry_bytes(const MixedCg * m);
 size_t mixed_row_bytes(const MixedCg * m);
 void mixed_destroy(MixedCg * m);

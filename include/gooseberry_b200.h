@@ -372,8 +372,9 @@ GOOSEBERRY_API int gb_cg_entry_bytes(const gb_cg_t * s, size_t * bytes);
 /* Bytes per row the solver's SpMV streams besides the entries: 4 (rowptr);
  * on a pattern matrix a pattern byte and the row's zero-padded values or
  * codes instead: 9 (8 codes), 33 (8 floats; MIXED, or exact floats), 49 or
- * 65 (6 or 8 doubles); 5 (rowptr and a pattern byte) for MIXED in builds
- * without its rows of values.  No reference counterpart. */
+ * 65 (6 or 8 doubles); 8, 12 or 16 for a symmetric pattern matrix of one to
+ * three distances above the diagonal past L2 (MIXED: its diagonals); 5 (rowptr
+ * and a pattern byte) for MIXED in builds without its rows of values.  No reference counterpart. */
 GOOSEBERRY_API int gb_cg_row_bytes(const gb_cg_t * s, size_t * bytes);
 
 /* ---- batched solve server (continuous batching) ---------------------------- */
