@@ -253,7 +253,8 @@ def run_cg_laplace(args, dist: Dist):
     xd = torch.empty_like(bd)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
 
-    # live per-kernel timing (first iterations of a real solve)
+    # live per-kernel timing (first iterations of a real solve); of a solve on
+    # the chip, its one kernel's two phases, each with its exchange between SMs
     ms_a, ms_b = S.profile(bd, iterations=40)
     # algorithmic bytes of the A kernel in the CSR layout (rowptr, column +
     # value per nonzero, r & p gathered once, p & Ap written); the kernel
@@ -318,9 +319,49 @@ def run_cg_laplace(args, dist: Dist):
     h2d = 4 * (n + 1) + 4 * nnz + 8 * nnz + 8 * n
     d2h = 8 * n
 
+    # a solve on the chip is one launch: the matrix's codes and every vector
+    # stay in shared memory and registers, so HBM sees 9 + 16 bytes a row once
+    # and the iterations' bytes (as the two-kernel form moves them) never leave
+    # the SMs
+    on_chip = results[-1].kernel_launches < iters
     peak, peak_src = hbm_peak()
     ach_a = bytes_a / (ms_a * 1e-3) / 1e9
     ach_a_stored = bytes_a_stored / (ms_a * 1e-3) / 1e9
+    if on_chip:
+        launch_ms = t_local / args.steps * 1e3
+        moved = (bytes_a + bytes_b) * iters
+        roofline = {
+            "bound": "latency (two exchanges between the SMs and a shared-memory row loop "
+                     "an iteration)",
+            "kernel": "cg_resident_kernel (the whole solve; vectors and value codes on the SMs)",
+            "achieved": moved / (launch_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
+            "frac": moved / (launch_ms * 1e-3) / 1e9 / peak,
+            "traffic": ncu_traffic("cg_resident_laplace1024"),
+            "bytes_per_launch": moved, "launch_ms": launch_ms, "peak_source": peak_src,
+            "bytes_per_launch_stored": S.row_bytes() * (n + 1) + 16 * n,
+            "on_chip": True, "l2_resident": False,
+            "frac_textbook_per_step": (bytes_textbook * iters * args.steps / t_local / 1e9)
+                                      / peak,
+        }
+    else:
+        roofline = {
+            "bound": "hbm",
+            "kernel": cg_a_kernel_name(entry_bytes, S.row_bytes()),
+            "achieved": ach_a, "peak": peak, "unit": "GB/s", "frac": ach_a / peak,
+            "traffic": ncu_traffic("cg_a_ell8_laplace1024" if ell8
+                                   else "cg_a_ellv_laplace1024" if entry_bytes == 0
+                                   else "cg_a_codec_laplace1024" if entry_bytes < 12
+                                   else "cg_a_row_laplace1024"),
+            "bytes_per_launch": bytes_a, "launch_ms": ms_a, "peak_source": peak_src,
+            "bytes_per_launch_stored": bytes_a_stored,
+            "achieved_stored": ach_a_stored, "frac_stored": ach_a_stored / peak,
+            # one iteration's working set (stored matrix + vectors) fits in
+            # the 126 MB L2, which the solve keeps it in (evict-last hints):
+            # the kernel's bytes mostly come from L2, not HBM
+            "l2_resident": bool(bytes_a_stored + 16 * n <= 126e6),
+            "frac_textbook_per_step": (bytes_textbook * iters * args.steps / t_local / 1e9)
+                                      / peak,
+        }
     out = {
         "metric": "CG solves/s (FP64, 2D 5-point Laplacian 1024x1024, rel-res 1e-8)",
         "value": rate,
@@ -345,24 +386,7 @@ def run_cg_laplace(args, dist: Dist):
             "l2": "flushed between steps (256 MB write, outside the timed events)",
             "parallelism": f"replicas x{dist.world}" if dist.world > 1 else "single GPU",
         },
-        "roofline": {
-            "bound": "hbm",
-            "kernel": cg_a_kernel_name(entry_bytes, S.row_bytes()),
-            "achieved": ach_a, "peak": peak, "unit": "GB/s", "frac": ach_a / peak,
-            "traffic": ncu_traffic("cg_a_ell8_laplace1024" if ell8
-                                   else "cg_a_ellv_laplace1024" if entry_bytes == 0
-                                   else "cg_a_codec_laplace1024" if entry_bytes < 12
-                                   else "cg_a_row_laplace1024"),
-            "bytes_per_launch": bytes_a, "launch_ms": ms_a, "peak_source": peak_src,
-            "bytes_per_launch_stored": bytes_a_stored,
-            "achieved_stored": ach_a_stored, "frac_stored": ach_a_stored / peak,
-            # one iteration's working set (stored matrix + vectors) fits in
-            # the 126 MB L2, which the solve keeps it in (evict-last hints):
-            # the kernel's bytes mostly come from L2, not HBM
-            "l2_resident": bool(bytes_a_stored + 16 * n <= 126e6),
-            "frac_textbook_per_step": (bytes_textbook * iters * args.steps / t_local / 1e9)
-                                      / peak,
-        },
+        "roofline": roofline,
         "kernels": {
             "cg_a_ms": ms_a, "cg_b_ms": ms_b,
             "cg_b_gbs": bytes_b / (ms_b * 1e-3) / 1e9,
