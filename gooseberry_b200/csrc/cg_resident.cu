@@ -483,6 +483,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
       }
     }
   }
+  if (a.arrived && blockIdx.x == 0 && tid == 0) a.out->t0 = res_ns();
   if (tid == 0) {
     sh.bad = 0;
     sh.cancel = 0;
@@ -741,6 +742,15 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
   }
   // any CTA that gave up marks the solve
   if (!ok && tid == 0) a.out->aborted = 1;
+  if (a.arrived) {  // every CTA's part of x and of the result, then `done`
+    __threadfence_system();
+    __syncthreads();
+    if (tid == 0 && atomicAdd(a.arrived, 1u) + 1 == gridDim.x) {
+      a.out->t1 = res_ns();
+      __threadfence_system();
+      *reinterpret_cast<volatile int *>(&a.out->done) = 1;
+    }
+  }
 }
 
 using ResKernel = void (*)(ResArgs);

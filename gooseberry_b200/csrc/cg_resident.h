@@ -50,6 +50,8 @@ struct ResResult {
   double rr, bnorm;
   unsigned epoch;  // all-reduces so far
   unsigned long long ns_a, ns_b;  // time in the two phases (a timed solve)
+  unsigned long long t0, t1;      // begin and end (with ResArgs::arrived)
+  int done;                       // written last (with ResArgs::arrived)
 };
 
 // ---- the solve kernel's arguments ------------------------------------------------
@@ -86,6 +88,8 @@ struct ResArgs {
   uint32_t epoch0;
   double tol;
   int timed;                      // report the phases' times
+  unsigned * arrived;             // may be null; 0 before: count the CTAs out, so that the last
+                                  // one reports `done` and no event has to follow the launch
 };
 
 // One solve's grid and kernel, from its size alone: matrix values in shared

@@ -100,11 +100,12 @@ constexpr size_t kMaxTiles = 1u << 20;
 // The batch streams every vector of every solve through L2 or HBM each
 // iteration; on the chip only the edge values and two sums cross L2.  Measured
 // (ms, all requests submitted and drained, batch -> here): 48 requests of 1k to
-// 262k rows 269 -> 92; 8 of them 204 -> 47; 20 of 1k to 65k rows 73 -> 20; 40 of
-// 1k to 16k rows, FP64, 30 -> 23.
+// 262k rows 269 -> 90; 8 of them 204 -> 48; 20 of 1k to 65k rows 73 -> 16; 40 of
+// 1k to 16k rows, FP64, 30 -> 10.
 //
 // Rows a CTA takes: more of them solve one request slower but leave SMs to
-// others.  2,048 up to 65,536 rows, past that 3,072 (the four cases above at
+// others.  2,048 up to 65,536 rows, past that 3,072 (the four cases, with at
+// most eight solves at once, 92, 47, 20 and 23 so, at
 // 2,048 throughout: 108, 47, 20, 23; at 3,072: 92, 48, 28, 27; at 1,024 large
 // systems do not fit).
 constexpr uint32_t srv_rows_per_cta(uint32_t n) { return n <= 65536 ? 2048 : 3072; }
@@ -683,7 +684,7 @@ struct SlotHost {
   double t_submit = 0.0, t_admit = 0.0;
   std::vector<SrvTile> tiles;
   // a solve on the chip
-  enum { kBatch, kWaiting, kRunning, kFinished } chip = kBatch;
+  enum { kBatch, kWaiting, kRunning, kChecking, kFinished } chip = kBatch;
   ResShape shape;
   SrvSlot dev{};                 // its device arrays (and the batch's, should it fall back)
   double * d = nullptr;          // refinement's correction (mixed)
@@ -750,7 +751,7 @@ struct gb_server {
   unsigned char * d_pin = nullptr;      // their device address
   std::vector<cudaStream_t> streams;    // made as they are needed
   std::vector<int> free_streams;
-  std::vector<cudaEvent_t> begin, end;  // per slot
+  std::vector<cudaEvent_t> end;  // per slot: behind its true residual
 };
 
 namespace gb {
@@ -819,8 +820,6 @@ void destroy_server(gb_server * s) {
     if (h.copied) cudaEventDestroy(h.copied);
   }
   for (auto & st : s->streams) cudaStreamDestroy(st);
-  for (auto & e : s->begin)
-    if (e) cudaEventDestroy(e);
   for (auto & e : s->end)
     if (e) cudaEventDestroy(e);
   cudaFree(s->d_ctl);
@@ -896,7 +895,6 @@ int create_server(const gb_server_config_t & cfg, gb_server * s) {
       cudaHostAllocMapped | cudaHostAllocPortable));
   std::memset(s->h_pin, 0, cfg.max_slots * kPinnedStride);
   GB_CUDA_TRY(cudaHostGetDevicePointer(&s->d_pin, s->h_pin, 0));
-  s->begin.assign(cfg.max_slots, nullptr);
   s->end.assign(cfg.max_slots, nullptr);
   GB_CUDA_TRY(cudaMalloc(&s->d_part, 2 * kMaxTiles * sizeof(double2)));
   s->slots.resize(cfg.max_slots);
@@ -1153,8 +1151,13 @@ int admit(gb_server & s, Request & q, uint32_t k) {
 }
 
 // Enqueue a solve on the chip for slot k (the first, or with rounds > 0 the
-// correction A d = b - A x), and behind it, in mixed mode, the true residual.
-// The caller holds its SMs.
+// correction A d = b - A x).  The caller holds its SMs.
+//
+// Nothing is queued behind the solve: the device's eight hardware queues are
+// shared by the streams, and work that waits for a solve blocks its queue, so
+// with an event behind each no more than eight solves ran at once.  The kernel
+// reports its end to the pinned block instead.  40 requests of 1k to 16k rows:
+// 23.4 -> 9.8 ms; 20 of 1k to 65k, mixed: 20.0 -> 16.4.
 int launch_on_chip(gb_server & s, uint32_t k) {
   SlotHost & h = s.slots[k];
   const SrvSlot & S = h.dev;
@@ -1169,8 +1172,6 @@ int launch_on_chip(gb_server & s, uint32_t k) {
     s.free_streams.pop_back();
   }
   cudaStream_t st = s.streams[h.stream];
-  if (!s.begin[k]) GB_CUDA_TRY(cudaEventCreate(&s.begin[k]));
-  if (!s.end[k]) GB_CUDA_TRY(cudaEventCreate(&s.end[k]));
   unsigned char * ctl = s.d_ctl + k * kCtlBytes;
   SrvPinned * pin = pinned(s, k);
   std::memset(&pin->res, 0, sizeof(pin->res));
@@ -1196,32 +1197,28 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   a.cancel = &pinned_dev(s, k)->cancel;
   a.out = &pinned_dev(s, k)->res;
   a.epoch0 = 2;
-  GB_CUDA_TRY(cudaEventRecord(s.begin[k], st));
+  a.arrived = reinterpret_cast<unsigned *>(ctl + kCtlFlag + 32);
   GB_TRY(resident_launch(h.shape, a, st));
-  if (s.mixed) {
-    if (h.rounds) GB_TRY(launch_add_to(h.n, h.d, S.x0, kSrvResidualGrid, st));
-    GB_TRY(launch_true_residual(h.n, S.rowptr, S.rowind, S.val64, S.b, S.x0, S.x1,
-        reinterpret_cast<double *>(ctl + kCtlPart), kSrvResidualGrid,
-        &pinned_dev(s, k)->rr_true, reinterpret_cast<unsigned *>(ctl + kCtlFlag + 16), st));
-  }
-  GB_CUDA_TRY(cudaEventRecord(s.end[k], st));
   h.chip = SlotHost::kRunning;
   return GOOSEBERRY_SUCCESS;
 }
 
-// Take slot k's ended solve: finished, to be corrected once more (mixed: the
-// recurrence met the tolerance before b - A x did), or back to the batch (a
-// wait inside it was given up).
+bool chip_done(gb_server & s, uint32_t k) {
+  return __atomic_load_n(&pinned(s, k)->res.done, __ATOMIC_ACQUIRE) != 0;
+}
+
+// Take slot k's ended solve: finished, or back to the batch (a wait inside it
+// was given up); in mixed mode its true residual is formed first.
 int collect_on_chip(gb_server & s, uint32_t k) {
   SlotHost & h = s.slots[k];
   const SrvPinned & pin = *pinned(s, k);
-  float ms = 0.f;
-  if (cudaEventElapsedTime(&ms, s.begin[k], s.end[k]) == cudaSuccess)  // its share of the device
-    s.stats.gpu_ms += ms * h.shape.args.ctas / std::max(1, s.sm_count);
+  s.stats.gpu_ms += (pin.res.t1 - pin.res.t0) * 1e-6 * h.shape.args.ctas /  // its share of the
+                    std::max(1, s.sm_count);                                // device
   resident_release(s.device, h.shape.args.ctas, chip_capacity(s));
-  s.free_streams.push_back(h.stream);
-  h.stream = -1;
   if (pin.res.aborted) {
+    GB_CUDA_TRY(cudaStreamSynchronize(s.streams[h.stream]));
+    s.free_streams.push_back(h.stream);
+    h.stream = -1;
     SrvSlot S = h.dev;
     if (s.mixed && h.nnz)
       GB_TRY(launch_round_f32(S.val64, const_cast<float *>(S.val32), h.nnz, s.stream));
@@ -1239,20 +1236,42 @@ int collect_on_chip(gb_server & s, uint32_t k) {
     h.bnorm = pin.res.bnorm;
     h.tol = h.dev.tol_rel * h.bnorm;
   }
-  h.chip = SlotHost::kFinished;
   if (s.mixed && h.bnorm != 0.0 && h.status != GB_CG_NONFINITE) {
-    ++h.rounds;
-    h.rnorm = std::sqrt(pin.rr_true);
-    if (!std::isfinite(h.rnorm)) {
-      h.status = GB_CG_NONFINITE;
-    } else if (h.status == GB_CG_CONVERGED && h.rnorm > h.tol) {
-      h.status = h.cancel ? GB_CG_CANCELLED : GB_CG_MAXITER;
-      if (h.iters < h.dev.niter && !h.cancel) h.chip = SlotHost::kWaiting;
-    } else if (h.status == GB_CG_MAXITER && h.rnorm <= h.tol) {
-      h.status = GB_CG_CONVERGED;
-    }
+    const SrvSlot & S = h.dev;
+    cudaStream_t st = s.streams[h.stream];
+    unsigned char * ctl = s.d_ctl + k * kCtlBytes;
+    if (!s.end[k]) GB_CUDA_TRY(cudaEventCreateWithFlags(&s.end[k], cudaEventDisableTiming));
+    if (h.rounds) GB_TRY(launch_add_to(h.n, h.d, S.x0, kSrvResidualGrid, st));
+    GB_TRY(launch_true_residual(h.n, S.rowptr, S.rowind, S.val64, S.b, S.x0, S.x1,
+        reinterpret_cast<double *>(ctl + kCtlPart), kSrvResidualGrid,
+        &pinned_dev(s, k)->rr_true, reinterpret_cast<unsigned *>(ctl + kCtlFlag + 16), st));
+    GB_CUDA_TRY(cudaEventRecord(s.end[k], st));
+    h.chip = SlotHost::kChecking;
+    return GOOSEBERRY_SUCCESS;
   }
+  s.free_streams.push_back(h.stream);
+  h.stream = -1;
+  h.chip = SlotHost::kFinished;
   return GOOSEBERRY_SUCCESS;
+}
+
+// Take slot k's true residual: the solve is finished, or to be corrected once
+// more (the recurrence met the tolerance before b - A x did).
+void collect_residual(gb_server & s, uint32_t k) {
+  SlotHost & h = s.slots[k];
+  s.free_streams.push_back(h.stream);
+  h.stream = -1;
+  h.chip = SlotHost::kFinished;
+  ++h.rounds;
+  h.rnorm = std::sqrt(pinned(s, k)->rr_true);
+  if (!std::isfinite(h.rnorm)) {
+    h.status = GB_CG_NONFINITE;
+  } else if (h.status == GB_CG_CONVERGED && h.rnorm > h.tol) {
+    h.status = h.cancel ? GB_CG_CANCELLED : GB_CG_MAXITER;
+    if (h.iters < h.dev.niter && !h.cancel) h.chip = SlotHost::kWaiting;
+  } else if (h.status == GB_CG_MAXITER && h.rnorm <= h.tol) {
+    h.status = GB_CG_CONVERGED;
+  }
 }
 
 // ---- the tile autotuner ------------------------------------------------------------
@@ -1489,15 +1508,29 @@ int step(gb_server & s, size_t * active, size_t * queued) {
   }
   // 0. collect the solves on the chip that have ended (a cancelled one stops
   //    within 64 iterations)
-  bool moved = false;
+  bool moved = false, asked = false;
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
-    if (!h.used || h.chip != SlotHost::kRunning) continue;
-    cudaError_t e = h.cancel ? cudaEventSynchronize(s.end[k]) : cudaEventQuery(s.end[k]);
-    if (e == cudaErrorNotReady) continue;
-    GB_CUDA_TRY(e);
-    GB_TRY(collect_on_chip(s, k));
-    moved = true;
+    if (h.used && h.chip == SlotHost::kRunning) {
+      if (h.cancel) GB_CUDA_TRY(cudaStreamSynchronize(s.streams[h.stream]));
+      if (!chip_done(s, k)) {
+        if (!asked) {  // a failed kernel reports nothing; its error shows on any stream
+          const cudaError_t e = cudaStreamQuery(s.stream);
+          if (e != cudaErrorNotReady) GB_CUDA_TRY(e);
+          asked = true;
+        }
+        continue;
+      }
+      GB_TRY(collect_on_chip(s, k));
+      moved = true;
+    }
+    if (h.used && h.chip == SlotHost::kChecking) {
+      const cudaError_t e = h.cancel ? cudaEventSynchronize(s.end[k]) : cudaEventQuery(s.end[k]);
+      if (e == cudaErrorNotReady) continue;
+      GB_CUDA_TRY(e);
+      collect_residual(s, k);
+      moved = true;
+    }
   }
   // 1. retire finished (or cancelled) solves: copy x out, free memory and
   //    the slot
@@ -1619,7 +1652,8 @@ int step(gb_server & s, size_t * active, size_t * queued) {
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     nact += s.slots[k].used ? 1 : 0;
     nbatch += s.slots[k].used && s.slots[k].chip == SlotHost::kBatch ? 1 : 0;
-    running += s.slots[k].used && s.slots[k].chip == SlotHost::kRunning ? 1 : 0;
+    running += s.slots[k].used && (s.slots[k].chip == SlotHost::kRunning ||
+                                   s.slots[k].chip == SlotHost::kChecking) ? 1 : 0;
   }
   if (launched && !nbatch) s.stats.steps += 1;
   // with nothing to do but wait for solves on the chip, wait for one (at most
@@ -1630,6 +1664,8 @@ int step(gb_server & s, size_t * active, size_t * queued) {
     while (!ended) {
       for (uint32_t k = 0; k < s.cfg.max_slots && !ended; ++k)
         if (s.slots[k].used && s.slots[k].chip == SlotHost::kRunning)
+          ended = chip_done(s, k);
+        else if (s.slots[k].used && s.slots[k].chip == SlotHost::kChecking)
           ended = cudaEventQuery(s.end[k]) != cudaErrorNotReady;
       const double w = std::chrono::duration<double, std::milli>(
           std::chrono::steady_clock::now() - w0).count();

@@ -145,3 +145,23 @@ def test_close_while_solves_run():
     b = torch.from_numpy(W.rhs(A.nrows, 1)).cuda()
     _, r = gb.CgSolver(M).solve(b, tol=1e-8)
     assert r.status == "converged"
+
+
+@pytest.mark.parametrize("mode", [gb.CG_F64, gb.CG_MIXED])
+def test_more_solves_at_once_than_hardware_queues(mode):
+    """60 requests of one or two CTAs each, all on the chip together: each ends
+    with the bits that it has alone, and the statistics count their time."""
+    reqs = [(k, W.diffusion_2d(24 + k, k)) for k in range(60)]
+    many = gb.Server(pool_bytes=1 << 29, max_slots=64, mode=mode)
+    for k, B in reqs:
+        many.submit(k, B, W.rhs(B.nrows, k), tol=1e-9, niter=20_000)
+    got = {r.id: r for r in many.drain()}
+    assert 0.0 < many.stats()["gpu_ms"] < 1e4
+    many.close()
+    one = gb.Server(pool_bytes=1 << 29, max_slots=1, mode=mode)
+    for k, B in reqs[::7]:
+        one.submit(k, B, W.rhs(B.nrows, k), tol=1e-9, niter=20_000)
+        r = one.drain()[0]
+        assert got[k].status == r.status == "converged" and got[k].iterations == r.iterations
+        assert np.array_equal(got[k].x, r.x)
+    one.close()
