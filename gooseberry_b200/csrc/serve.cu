@@ -104,15 +104,14 @@ constexpr size_t kMaxTiles = 1u << 20;
 // 1k to 16k rows, FP64, 30 -> 10.
 //
 // Rows a CTA takes: more of them solve one request slower but leave SMs to
-// others.  2,048 up to 65,536 rows, past that 3,072 (the four cases, with at
-// most eight solves at once, 92, 47, 20 and 23 so, at
-// 2,048 throughout: 108, 47, 20, 23; at 3,072: 92, 48, 28, 27; at 1,024 large
-// systems do not fit).
+// others.  2,048 up to 65,536 rows, past that 3,072 (the four cases, when at
+// most eight solves ran at once, so: 92, 47, 20, 23; at 2,048 throughout: 108,
+// 47, 20, 23; at 3,072: 92, 48, 28, 27; at 1,024 large systems do not fit).
 constexpr uint32_t srv_rows_per_cta(uint32_t n) { return n <= 65536 ? 2048 : 3072; }
 constexpr unsigned kSrvResidualGrid = 64;  // CTAs of the true-residual kernel
 constexpr uint32_t kSrvPatMax = 256;
 // Device control block of a slot: fixed-point words, tagged partials, abort
-// flag and ticket, residual partials.
+// flag, ticket and count of CTAs that are out, residual partials.
 constexpr size_t kCtlBox = 256;
 constexpr size_t kCtlFlag = kCtlBox + 2 * kResMaxCtas * 16;
 constexpr size_t kCtlPart = kCtlFlag + 64;
