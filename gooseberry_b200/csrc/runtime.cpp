@@ -186,9 +186,12 @@ void pinned_slot_free(void * host) {
 // sent as soon as it is there.  Pieces are 1 MiB and every thread alternates
 // between two slots: 16 MiB of pinned memory per device, kept for the life of
 // the process and used by one upload at a time (another one meanwhile takes the
-// driver's path).  From 24 MiB up: below, starting the threads (0.3 ms) takes
-// what they save (19 MB of CSR arrays: 1.58 ms by the driver, 1.75 so; 196 MB:
-// 18.8 and 7.2).
+// driver's path).  cudaStreamPerThread names another stream in every thread, so
+// for that handle the pieces go through a stream of the slots' own, between two
+// events that the calling thread puts on its stream.
+//
+// From 24 MiB up: below, starting the threads (0.3 ms) takes what they save
+// (19 MB of CSR arrays: 1.58 ms by the driver, 1.75 so; 196 MB: 18.8 and 7.2).
 namespace {
 constexpr size_t kUpPiece = 1 << 20;
 constexpr int kUpThreads = 8;
@@ -198,6 +201,8 @@ struct UploadSlots {
   bool made = false, failed = false;
   void * pinned[kUpThreads][2] = {};
   cudaEvent_t sent[kUpThreads][2] = {};
+  cudaStream_t own = nullptr;  // for cudaStreamPerThread
+  cudaEvent_t edge = nullptr;
 };
 std::mutex g_up_mu;
 std::map<int, UploadSlots *> g_up;
@@ -220,6 +225,12 @@ bool make_slots(UploadSlots & u) {
         return false;
       }
     }
+  if (cudaStreamCreateWithFlags(&u.own, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&u.edge, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFreeHost(block);
+    return false;
+  }
   u.failed = false;
   return u.made = true;
 }
@@ -249,6 +260,11 @@ int upload(void * dst, const void * src, size_t bytes, cudaStream_t s) {
     GB_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
     return GOOSEBERRY_SUCCESS;
   }
+  const cudaStream_t via = s == cudaStreamPerThread ? u->own : s;  // the same in every thread
+  if (via != s) {
+    GB_CUDA_TRY(cudaEventRecord(u->edge, s));
+    GB_CUDA_TRY(cudaStreamWaitEvent(via, u->edge, 0));
+  }
   const size_t pieces = (bytes + kUpPiece - 1) / kUpPiece;
   std::atomic<size_t> next{0};
   std::atomic<int> err{cudaSuccess};
@@ -262,8 +278,8 @@ int upload(void * dst, const void * src, size_t bytes, cudaStream_t s) {
       if (e != cudaSuccess) break;
       std::memcpy(u->pinned[t][q], static_cast<const char *>(src) + at, len);
       e = cudaMemcpyAsync(static_cast<char *>(dst) + at, u->pinned[t][q], len,
-          cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess) e = cudaEventRecord(u->sent[t][q], s);
+          cudaMemcpyHostToDevice, via);
+      if (e == cudaSuccess) e = cudaEventRecord(u->sent[t][q], via);
     }
     if (e != cudaSuccess) err.store(e);
   };
@@ -279,6 +295,10 @@ int upload(void * dst, const void * src, size_t bytes, cudaStream_t s) {
   work(0);
   for (auto & h : helpers) h.join();
   GB_CUDA_TRY(static_cast<cudaError_t>(err.load()));
+  if (via != s) {
+    GB_CUDA_TRY(cudaEventRecord(u->edge, via));
+    GB_CUDA_TRY(cudaStreamWaitEvent(s, u->edge, 0));
+  }
   return GOOSEBERRY_SUCCESS;
 }
 
