@@ -56,6 +56,7 @@ SCHED_NAMES = {0: "auto", 1: "thread", 2: "group4", 3: "group8", 4: "warp", 5: "
 CG_F64, CG_MIXED = 0, 1
 CG_PERSISTENT = 0x100
 CG_PLAIN_ENTRIES = 0x200
+CHIP_FAULT_NONE, CHIP_FAULT_MISSING, CHIP_FAULT_LATE = 0, 1, 2
 CG_STATUS = {0: "converged", 1: "maxiter", 2: "breakdown", 3: "nonfinite", 4: "cancelled",
              5: "timeout"}
 
@@ -144,6 +145,7 @@ SIGNATURES = {
     "gb_cg_row_bytes": (_i, [_vp, _vp]),
     "gb_cg_cancel": (_i, [_vp]),
     "gb_cg_set_barrier_fault": (_i, [_vp, C.c_int, C.c_uint]),
+    "gb_cg_set_chip_fault": (_i, [_vp, C.c_int, C.c_uint]),
     "gb_server_cancel": (_i, [_vp, C.c_uint64]),
     "gb_server_stats": (_i, [_vp, _vp]),
     "gb_server_tuned_tile_rows": (_i, [C.c_int, C.c_uint32, C.c_uint32, _vp]),
@@ -696,6 +698,14 @@ class CgSolver:
         (status "timeout"); ``drop_cta < 0`` turns it off."""
         _check(lib().gb_cg_set_barrier_fault(self._h, int(drop_cta), int(limit_ms)),
                "gb_cg_set_barrier_fault")
+
+    def set_chip_fault(self, fault: int = CHIP_FAULT_NONE, limit_ms: int = 0):
+        """Failure-path hook of solves on the chip (``gb_cg_set_chip_fault``): a CTA
+        of the following solves is missing (``CHIP_FAULT_MISSING``) or late
+        (``CHIP_FAULT_LATE``), so they are given up after ``limit_ms`` (0: the 2 s
+        default) and run by the graph-replayed kernels."""
+        _check(lib().gb_cg_set_chip_fault(self._h, int(fault), int(limit_ms)),
+               "gb_cg_set_chip_fault")
 
     def entry_bytes(self) -> int:
         """Bytes per matrix entry the solver's SpMV streams (12 = plain CSR)."""

@@ -1880,6 +1880,15 @@ int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned limit_ms) {
   return GOOSEBERRY_SUCCESS;
 }
 
+int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms) {
+  GB_CHECK_INPUT(s != nullptr, "solver is NULL");
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_LATE, "unknown fault %d",
+      fault);
+  GB_CHECK_INPUT(s->resident && gb::resident_set_fault(s->resident, fault, limit_ms),
+      "the fault applies to solves on the chip by more than one CTA");
+  return GOOSEBERRY_SUCCESS;
+}
+
 int gb_cg_entry_bytes(const gb_cg_t * s, size_t * bytes) {
   GB_CHECK_INPUT(s != nullptr && bytes != nullptr, "NULL argument");
   *bytes = s->mixed ? mixed_entry_bytes(s->mixed)

@@ -158,15 +158,22 @@ __device__ __forceinline__ double tagged_value(const ulonglong2 & m) {
 }
 
 // Every 256 polls: has some CTA given up, or is it time to?
-__device__ __forceinline__ bool res_give_up(int * abort_flag, unsigned polls,
+__device__ __forceinline__ bool res_give_up(const ResArgs & a, unsigned polls,
     unsigned long long * t0) {
   if (polls & 255u) return false;
-  if (*reinterpret_cast<volatile int *>(abort_flag)) return true;
+  if (*reinterpret_cast<volatile int *>(a.abort_flag)) return true;
   const unsigned long long now = res_ns();
   if (*t0 == 0) *t0 = now;
-  if (now - *t0 <= kResWaitNs) return false;
-  atomicExch(abort_flag, 1);
+  if (now - *t0 <= a.wait_ns) return false;
+  atomicExch(a.abort_flag, 1);
   return true;
+}
+
+// A test's late CTA.
+__device__ __forceinline__ void res_be_late(unsigned long long ns) {
+  const unsigned long long end = res_ns() + ns;
+#pragma unroll 1
+  for (unsigned k = 0; k < (1u << 24) && res_ns() < end; ++k) __nanosleep(2000);
 }
 
 __device__ __forceinline__ double warp_allsum(double v) {
@@ -178,7 +185,8 @@ __device__ __forceinline__ double warp_allsum(double v) {
 struct ResShared {
   double red[32];
   double total;
-  int bad;         // a wait in this CTA was given up
+  int bad;         // a wait for a neighbour's r was given up
+  int leave;       // that, or a wait of this all-reduce's: what all threads go by
   int cancel;      // the host asked to stop (CTA 0's view, as of this all-reduce)
   int cancel_req;  // CTA 0: what it will send
   double bnorm, tol, rr_far;
@@ -193,8 +201,8 @@ struct ResSums {
 
 // Every CTA's `v` by tagged messages, added in CTA order: lane l adds those of
 // CTAs l, l + 32, ..., then the warp tree.  All lanes of warp 0 call it.
-__device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResShared & sh, ResSums & st,
-    uint32_t epoch, double v, int * cancel) {
+__device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResSums & st,
+    uint32_t epoch, double v, int * cancel, int * bad) {
   const int lane = threadIdx.x & 31;
   ulonglong2 * const box = a.box + (st.tagged++ & 1) * a.ctas;
   const uint32_t tag = epoch << 1;
@@ -206,8 +214,8 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResShared & 
   for (uint32_t c = lane; c < a.ctas; c += 32) {
     ulonglong2 m = tagged_load(box + c);
     while (!tag_is(make_ulonglong2(m.x & kNoCancel, m.y & kNoCancel), tag)) {
-      if (res_give_up(a.abort_flag, ++polls, &t0)) {
-        sh.bad = 1;
+      if (res_give_up(a, ++polls, &t0)) {
+        *bad = 1;
         break;
       }
       m = tagged_load(box + c);
@@ -216,6 +224,7 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResShared & 
     if (c == 0) *cancel = static_cast<int>((m.x >> 32) & 1u);
   }
   *cancel = __shfl_sync(0xffffffffu, *cancel, 0);
+  *bad = __any_sync(0xffffffffu, *bad);
   return warp_allsum(acc);
 }
 
@@ -228,8 +237,8 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResShared & 
 // fit or the sum is so much smaller than `prev` that the cut-off bits
 // (2^(E - 131) a CTA) would show in its 53.
 template <class S>
-__device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResShared & sh, ResSums & st,
-    double v, double prev, int * cancel, double * total, S && sent) {
+__device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResSums & st, double v,
+    double prev, int * cancel, int * bad, double * total, S && sent) {
   const int lane = threadIdx.x & 31;
   const int e = ((__double2hiint(prev) >> 20) & 0x7ff) - 1023 + 40;
   const bool odd = st.fixed++ & 1;
@@ -260,8 +269,8 @@ __device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResShared & sh,
     if (lane < 3) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(cur) : "l"(w) : "memory");
     const bool all = lane >= 3 || static_cast<uint32_t>((cur - seen) >> 56) == a.ctas;
     if (__all_sync(0xffffffffu, all)) break;
-    if (__any_sync(0xffffffffu, res_give_up(a.abort_flag, polls, &t0))) {
-      sh.bad = 1;
+    if (__any_sync(0xffffffffu, res_give_up(a, polls, &t0))) {
+      *bad = 1;
       break;
     }
   }
@@ -286,9 +295,11 @@ __device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResShared & sh,
 }
 
 // Sum of every CTA's `local` (over its threads), the same bits in every CTA.
-// `prev`: a sum of about this size, the same in every CTA (0: unknown).  Warps 1.. run `hidden` while warp 0 exchanges the sums, and warp 0
-// runs `sent` between its send and its wait.  Returns false when a wait was
-// given up.
+// `prev`: a sum of about this size, the same in every CTA (0: unknown).  Warps
+// 1.. run `hidden` while warp 0 exchanges the sums, and warp 0
+// runs `sent` between its send and its wait.  Returns false, in every thread of
+// the CTA alike, when a wait was given up before the sum was complete (a wait
+// of `hidden` that is given up later is told by the next all-reduce).
 template <int T, class F, class S>
 __device__ __forceinline__ bool res_allreduce(const ResArgs & a, ResShared & sh, ResSums & st,
     uint32_t & epoch, double local, double prev, F && hidden, S && sent, double * total) {
@@ -299,27 +310,28 @@ __device__ __forceinline__ bool res_allreduce(const ResArgs & a, ResShared & sh,
   if (warp == 0) {
     const double v = warp_allsum(lane < T / 32 ? sh.red[lane] : 0.0);
     double sum = v;
-    int cancel = sh.cancel_req;
+    int cancel = sh.cancel_req, bad = sh.bad;
     if (a.ctas > 1) {
       // (the bounds keep the fixed point's unit and the sum normal)
       const bool known = prev > 0x1p-960 && prev < INFINITY;
       const int asked = cancel;
       if (!known) sent();
-      if (!known || !res_sum_fixed(a, sh, st, v, prev, &cancel, &sum, sent)) {
+      if (!known || !res_sum_fixed(a, st, v, prev, &cancel, &bad, &sum, sent)) {
         cancel = asked;
-        sum = res_sum_tagged(a, sh, st, epoch, v, &cancel);
+        sum = res_sum_tagged(a, st, epoch, v, &cancel, &bad);
       }
     }
     if (lane == 0) {
       sh.total = sum;
       sh.cancel = cancel;
+      sh.leave = bad;
     }
   } else {
     hidden();
   }
   __syncthreads();
   *total = sh.total;
-  return sh.bad == 0;
+  return sh.leave == 0;
 }
 
 // One thread's cached view of a row pattern (and, for RES_CLASS, its values):
@@ -538,7 +550,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
         const uint32_t j = j0 + u * step, g = row_of(j);
         if (j < nh && g < a.n) {
           while (!tag_is(m[u], epoch)) {
-            if (res_give_up(a.abort_flag, ++polls, &t0)) {
+            if (res_give_up(a, ++polls, &t0)) {
               sh.bad = 1;
               break;
             }
@@ -707,8 +719,10 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
           else res_x_update(a.x + lo, po, alpha, tid - 32, nloc, kHidden);
           prefetch_halo();
           // the host's flag costs a trip over PCIe, so it is read now and then
-          if (blockIdx.x == 0 && tid == T - 1 && (it & 63) == 0)
+          if (blockIdx.x == 0 && tid == T - 1 && (it & 63) == 0) {
+            if (it && a.late_ns) res_be_late(a.late_ns);
             sh.cancel_req = *reinterpret_cast<const volatile int *>(a.cancel) != 0;
+          }
         }, publish, &rr_new)) {
       ok = false;
       break;
@@ -741,7 +755,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     a.out->ns_b = t_b;
   }
   // any CTA that gave up marks the solve
-  if (!ok && tid == 0) a.out->aborted = 1;
+  if ((!ok || sh.bad) && tid == 0) a.out->aborted = 1;
   if (a.arrived) {  // every CTA's part of x and of the result, then `done`
     __threadfence_system();
     __syncthreads();
@@ -849,7 +863,14 @@ struct ResidentCg {
   ResResult * out_d = nullptr;
   RowClasses classes;
   uint32_t epoch = 0;        // all-reduces so far; 0: tags have to be cleared
+  int fault = GB_CHIP_FAULT_NONE;  // for tests
 };
+
+// The grid of a solve (a test's missing CTA is the last one: the others wait for
+// its part of the sums and for its edge values).
+static unsigned resident_grid(const ResArgs & g, int fault) {
+  return g.ctas - (fault == GB_CHIP_FAULT_MISSING && g.ctas > 1 ? 1u : 0u);
+}
 
 void resident_destroy(ResidentCg * s) {
   if (!s) return;
@@ -886,6 +907,7 @@ int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sm
     out->args.halo = halo;
     out->args.ctas = ctas;
     out->args.ncode = npat;
+    resident_set_waits(&out->args, GB_CHIP_FAULT_NONE, 0);
     out->args.at = ResPlaces{1, ctas > 1 && need(ResPlaces{1, 1}) <= room ? 1 : 0};
     out->smem = need(out->args.at);
     out->threads = kResThreads;
@@ -912,7 +934,7 @@ int resident_preload() {
 
 int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream) {
   void * kargs[] = {&args};
-  GB_CUDA_TRY(cudaLaunchCooperativeKernel(sh.fn, dim3(args.ctas), dim3(sh.threads), kargs, sh.smem,
+  GB_CUDA_TRY(cudaLaunchCooperativeKernel(sh.fn, dim3(resident_grid(args, sh.fault)), dim3(sh.threads), kargs, sh.smem,
       stream));
   return GOOSEBERRY_SUCCESS;
 }
@@ -978,6 +1000,7 @@ int resident_create(const gb_csr & a, const ResidentIn & in, double * x, Residen
   g.pat_off = in.pat->off;
   g.ncode = in.pat->npat;
   g.x = x;
+  resident_set_waits(&g, GB_CHIP_FAULT_NONE, 0);
   const int k = static_cast<int>((rows + threads - 1) / threads);
   int src = RES_CSR;
   if (!in.plain) {
@@ -1043,6 +1066,18 @@ int resident_create(const gb_csr & a, const ResidentIn & in, double * x, Residen
   return GOOSEBERRY_SUCCESS;
 }
 
+void resident_set_waits(ResArgs * g, int fault, unsigned limit_ms) {
+  g->wait_ns = limit_ms ? limit_ms * 1000000ull : kResWaitNs;
+  g->late_ns = fault == GB_CHIP_FAULT_LATE ? 2 * g->wait_ns : 0;
+}
+
+bool resident_set_fault(ResidentCg * s, int fault, unsigned limit_ms) {
+  if (fault != GB_CHIP_FAULT_NONE && s->args.ctas < 2) return false;
+  s->fault = fault;
+  resident_set_waits(&s->args, fault, limit_ms);
+  return true;
+}
+
 int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relative,
     unsigned long long niter, double * dhist, unsigned long long hist_len,
     const int * cancel_h, const int * cancel_d, bool timed, cudaStream_t stream,
@@ -1076,7 +1111,7 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
   }
   void * kargs[] = {&g};
   cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(s->fn),
-      dim3(g.ctas), dim3(s->threads), kargs, s->smem, stream);
+      dim3(resident_grid(g, s->fault)), dim3(s->threads), kargs, s->smem, stream);
   const cudaError_t e2 = cudaStreamSynchronize(stream);
   if (units) resident_release(s->a->device, units, s->capacity);
   if (e == cudaSuccess) e = e2;

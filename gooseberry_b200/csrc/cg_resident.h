@@ -88,6 +88,8 @@ struct ResArgs {
   uint32_t epoch0;
   double tol;
   int timed;                      // report the phases' times
+  unsigned long long wait_ns;     // a wait that lasts longer is given up
+  unsigned long long late_ns;     // for tests: CTA 0 is that late after iteration 64
   unsigned * arrived;             // may be null; 0 before: count the CTAs out, so that the last
                                   // one reports `done` and no event has to follow the launch
 };
@@ -100,7 +102,10 @@ struct ResShape {
   const void * fn = nullptr;
   size_t smem = 0;
   int threads = 0;
+  int fault = GB_CHIP_FAULT_NONE;  // for tests
 };
+// Sets the limit of a solve's waits (0: the usual one) and, for tests, a fault.
+void resident_set_waits(ResArgs * g, int fault, unsigned limit_ms);
 int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,
     ResShape * out);
 // Load every kernel that resident_shape may choose.  A kernel is otherwise
@@ -151,6 +156,11 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
     unsigned long long niter, double * dhist, unsigned long long hist_len,
     const int * cancel_h, const int * cancel_d, bool timed, cudaStream_t stream,
     ResOutcome * res);
+
+// For tests of the give-up path: what the following solves do (GB_CHIP_FAULT_*)
+// and the limit of their waits in ms (0: the usual one); false if the solve has
+// one CTA, which waits for nobody.
+bool resident_set_fault(ResidentCg * s, int fault, unsigned limit_ms);
 
 // SMs of a device shared by the grids whose CTAs wait for one another; false
 // if `cancel` (host, may be null) was set before the SMs were free.

@@ -347,6 +347,21 @@ GOOSEBERRY_API int gb_cg_cancel(gb_cg_t * s);
  * device stays usable.  No reference counterpart (cgd runs on the host). */
 GOOSEBERRY_API int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned limit_ms);
 
+/* Failure-path hook for solves on the chip, for tests of their bounded waits:
+ * in the following solves the last CTA does not start (MISSING), or CTA 0 is
+ * late after iteration 64 by twice the wait limit (LATE).  The other CTAs give
+ * up when the limit is over, raise the abort flag and leave (as a late one then
+ * does), and the call runs the solve by the graph-replayed kernels and returns
+ * their result.  `limit_ms` sets the limit (0: 2000).  Nothing waits without
+ * one, so the device stays usable.  Refused for a solver that does not solve on
+ * the chip, or that does on one CTA.  No reference counterpart. */
+typedef enum gb_chip_fault {
+  GB_CHIP_FAULT_NONE = 0,
+  GB_CHIP_FAULT_MISSING = 1,
+  GB_CHIP_FAULT_LATE = 2
+} gb_chip_fault_t;
+GOOSEBERRY_API int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms);
+
 /*
  * Measurement hook: start a solve of A x = b and run its first `iterations`
  * iterations launch by launch, timing every launch with CUDA events on
