@@ -154,6 +154,7 @@ SIGNATURES = {
     "gb_server_submit": (_i, [_vp, C.c_uint64, _u32, _vp, _vp, _vp, _vp, _vp, _d, _sz]),
     "gb_server_step": (_i, [_vp, _vp, _vp]),
     "gb_server_poll": (_i, [_vp, _vp, _sz, _vp]),
+    "gb_server_set_chip_fault": (_i, [_vp, C.c_int, C.c_uint]),
     "gb_server_clock": (_d, [_vp]),
 }
 
@@ -827,6 +828,12 @@ class Server:
         """Cancel a queued or resident request (``gb_server_cancel``); it is
         reported by ``poll`` with status "cancelled" (x_out untouched)."""
         _check(lib().gb_server_cancel(self._h, int(rid)), "gb_server_cancel")
+
+    def set_chip_fault(self, fault: int = CHIP_FAULT_NONE, limit_ms: int = 0):
+        """``CgSolver.set_chip_fault`` for the requests solved on the chip from now
+        on (``gb_server_set_chip_fault``); given up, they go to the batch."""
+        _check(lib().gb_server_set_chip_fault(self._h, int(fault), int(limit_ms)),
+               "gb_server_set_chip_fault")
 
     def clock(self) -> float:
         return float(lib().gb_server_clock(self._h))

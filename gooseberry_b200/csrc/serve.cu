@@ -751,6 +751,8 @@ struct gb_server {
   std::vector<cudaStream_t> streams;    // made as they are needed
   std::vector<int> free_streams;
   std::vector<cudaEvent_t> end;  // per slot: behind its true residual
+  int fault = GB_CHIP_FAULT_NONE;  // for tests (gb_server_set_chip_fault)
+  unsigned fault_limit_ms = 0;
 };
 
 namespace gb {
@@ -1175,6 +1177,7 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   SrvPinned * pin = pinned(s, k);
   std::memset(&pin->res, 0, sizeof(pin->res));
   pin->rr_true = 0.0;
+  __atomic_store_n(&pin->cancel, 0, __ATOMIC_RELEASE);  // a request to stop belongs to one launch
   GB_CUDA_TRY(cudaStreamWaitEvent(st, h.copied, 0));
   GB_CUDA_TRY(cudaMemsetAsync(ctl, 0, kCtlBytes, st));
   GB_CUDA_TRY(cudaMemsetAsync(h.r_edge, 0, 16ull * h.n, st));
@@ -1197,6 +1200,8 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   a.out = &pinned_dev(s, k)->res;
   a.epoch0 = 2;
   a.arrived = reinterpret_cast<unsigned *>(ctl + kCtlFlag + 32);
+  resident_set_waits(&a, s.fault, s.fault_limit_ms);
+  h.shape.fault = s.fault;
   GB_TRY(resident_launch(h.shape, a, st));
   h.chip = SlotHost::kRunning;
   return GOOSEBERRY_SUCCESS;
@@ -1568,7 +1573,6 @@ int step(gb_server & s, size_t * active, size_t * queued) {
         GB_CUDA_TRY(cudaEventSynchronize(h.copied));  // (cancelled before it was launched)
         cudaEventDestroy(h.copied);
       }
-      __atomic_store_n(&pinned(s, k)->cancel, 0, __ATOMIC_RELEASE);
     }
     res.t_submit = h.t_submit;
     res.t_admit = h.t_admit;
@@ -1757,6 +1761,15 @@ int gb_server_poll(gb_server_t * s, gb_server_result_t * out, size_t max, size_t
 int gb_server_cancel(gb_server_t * s, uint64_t id) {
   GB_CHECK_INPUT(s != nullptr, "server is NULL");
   return gb::cancel(*s, id);
+}
+
+int gb_server_set_chip_fault(gb_server_t * s, int fault, unsigned limit_ms) {
+  GB_CHECK_INPUT(s != nullptr, "server is NULL");
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_LATE, "unknown fault %d",
+      fault);
+  s->fault = fault;
+  s->fault_limit_ms = limit_ms;
+  return GOOSEBERRY_SUCCESS;
 }
 
 double gb_server_clock(const gb_server_t * s) { return s ? gb::now_s(*s) : 0.0; }

@@ -469,6 +469,11 @@ GOOSEBERRY_API int gb_server_poll(gb_server_t * s, gb_server_result_t * out, siz
  * has no server, so no counterpart. */
 GOOSEBERRY_API int gb_server_cancel(gb_server_t * s, uint64_t id);
 
+/* gb_cg_set_chip_fault for the requests that the server solves on the chip from
+ * now on; those that are given up are solved by the batch.  No reference
+ * counterpart. */
+GOOSEBERRY_API int gb_server_set_chip_fault(gb_server_t * s, int fault, unsigned limit_ms);
+
 /* Seconds since the server was created (the clock of the result stamps). */
 GOOSEBERRY_API double gb_server_clock(const gb_server_t * s);
 
