@@ -1530,6 +1530,23 @@ int launch_add_to(size_t n, const double * d, double * x, unsigned grid, cudaStr
 
 namespace {
 
+// ||v|| of a device vector, to the host.
+int host_norm(size_t n, const double * v, double * norm, cudaStream_t stream) {
+  double * d = nullptr;
+  double rr = 0.0;
+  GB_TRY(scratch_alloc(reinterpret_cast<void **>(&d), sizeof(double), stream));
+  int rc = gb_dot_f64(n, v, v, d, stream);
+  cudaError_t e = cudaSuccess;
+  if (rc == GOOSEBERRY_SUCCESS)
+    e = cudaMemcpyAsync(&rr, d, sizeof(double), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  scratch_free(d, stream);
+  GB_TRY(rc);
+  GB_CUDA_TRY(e);
+  *norm = std::sqrt(rr);
+  return GOOSEBERRY_SUCCESS;
+}
+
 // A solve on the chip.  *done = false: a wait inside it was given up (some
 // other program holds SMs), and the graph path has to run the solve.
 //
@@ -1565,7 +1582,13 @@ int solve_resident(gb_cg * s, const double * b, double * x, double tol, int tol_
       const unsigned g = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(
           (s->n + kVecBlock - 1) / kVecBlock, static_cast<size_t>(s->a->sm_count) * 4)));
       if (out.cancelled_waiting) {
-        if (rounds == 0) GB_CUDA_TRY(cudaMemsetAsync(x, 0, s->n * sizeof(double), stream));
+        // x and its residual stay those of the last round; before the first, x = 0
+        if (rounds == 0) {
+          GB_CUDA_TRY(cudaMemsetAsync(x, 0, s->n * sizeof(double), stream));
+          GB_TRY(host_norm(s->n, b, &bnorm, stream));
+          rnorm = bnorm;
+        }
+        break;
       } else if (rounds == 0) {
         bnorm = r.bnorm;
         if (tol_relative) tol *= bnorm;
@@ -1577,7 +1600,7 @@ int solve_resident(gb_cg * s, const double * b, double * x, double tol, int tol_
       }
       iters += r.iter;
       rnorm = std::sqrt(r.rr);
-      if (!refine || out.cancelled_waiting || status == GB_CG_NONFINITE || bnorm == 0.0) break;
+      if (!refine || status == GB_CG_NONFINITE || bnorm == 0.0) break;
       GB_TRY(launch_true_residual(static_cast<uint32_t>(s->n), s->a->rowptr, s->a->rowind,
           s->a->val64, b, s->xsum, s->r, s->partial_a, g, s->rr_true_d, s->ticket, stream));
       GB_CUDA_TRY(cudaStreamSynchronize(stream));
