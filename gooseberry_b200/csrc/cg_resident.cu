@@ -796,56 +796,102 @@ ResKernel res_kernel_s(int src, int threads, int k) {
 //
 // A resident grid's CTAs wait for one another, so all of them must get an SM.
 // Solves of one process on one device share its SMs through this count: a
-// solve takes as many units as it has CTAs and waits while they are not free.
+// solve holds as many units as it has CTAs and waits while they are not free.
+// A holder that nobody waits for on the host (the solve server's) names the
+// word in which its kernel reports its end: whoever needs SMs takes those of
+// ended holders back, so nobody depends on the holder's owner to look.
 struct ResGate {
+  struct Held {
+    unsigned long long id;
+    unsigned units;
+    const int * done;  // may be null
+  };
+  struct Device {
+    unsigned used = 0;
+    std::vector<Held> held;
+    unsigned long long next = 0, serving = 0;  // first come, first served
+  };
   std::mutex mu;
   std::condition_variable cv;
-  std::map<int, unsigned> used;       // per device
-  std::map<int, unsigned long long> next, serving;  // first come, first served
+  std::map<int, Device> devices;
+  unsigned long long last_id = 0;
 };
 ResGate & gate() {
   static ResGate g;
   return g;
 }
 
+// Drop holders that `gone` names.  The gate is locked.
+template <class F>
+void gate_drop(ResGate & g, ResGate::Device & d, F && gone) {
+  for (size_t k = 0; k < d.held.size();)
+    if (gone(d.held[k])) {
+      d.used -= d.held[k].units;
+      d.held.erase(d.held.begin() + k);
+      g.cv.notify_all();
+    } else {
+      ++k;
+    }
+}
+
+// A holder's id if its units are free now, else 0.  The gate is locked.
+unsigned long long gate_take(ResGate & g, ResGate::Device & d, unsigned units, unsigned capacity,
+    const int * done) {
+  gate_drop(g, d, [](const ResGate::Held & h) {
+    return h.done && __atomic_load_n(h.done, __ATOMIC_ACQUIRE);
+  });
+  units = std::min(units, capacity);
+  if (d.used + units > capacity) return 0;
+  d.held.push_back({++g.last_id, units, done});
+  d.used += units;
+  return g.last_id;
+}
+
 }  // namespace
 
-bool resident_acquire(int device, unsigned ctas, unsigned capacity, const int * cancel) {
+unsigned long long resident_acquire(int device, unsigned ctas, unsigned capacity,
+    const int * cancel, unsigned long long limit_ns, bool * cancelled) {
   ResGate & g = gate();
   std::unique_lock<std::mutex> lk(g.mu);
-  const unsigned long long mine = g.next[device]++;
+  ResGate::Device & d = g.devices[device];
+  const unsigned long long mine = d.next++;
+  *cancelled = false;
+  std::chrono::steady_clock::time_point since{};
+  unsigned long long id = 0;
   for (;;) {
-    const bool turn = g.serving[device] == mine;
-    if (turn && g.used[device] + std::min(ctas, capacity) <= capacity) break;
-    // a cancelled wait still takes its turn, so that the queue moves on
-    if (turn && cancel && __atomic_load_n(cancel, __ATOMIC_ACQUIRE)) {
-      ++g.serving[device];
-      g.cv.notify_all();
-      return false;
+    if (d.serving == mine) {
+      if ((id = gate_take(g, d, ctas, capacity, nullptr)) != 0) break;
+      // a wait that is given up still takes its turn, so that the queue moves on
+      if (cancel && __atomic_load_n(cancel, __ATOMIC_ACQUIRE)) {
+        *cancelled = true;
+        break;
+      }
+      const auto now = std::chrono::steady_clock::now();
+      if (since.time_since_epoch().count() == 0) since = now;
+      if (static_cast<unsigned long long>(
+              std::chrono::duration_cast<std::chrono::nanoseconds>(now - since).count()) >
+          limit_ns)
+        break;
     }
-    g.cv.wait_for(lk, std::chrono::milliseconds(2));
+    g.cv.wait_for(lk, std::chrono::microseconds(200));  // an ended kernel notifies nobody
   }
-  ++g.serving[device];
-  g.used[device] += std::min(ctas, capacity);
+  ++d.serving;
   g.cv.notify_all();
-  return true;
+  return id;
 }
 
-bool resident_try_acquire(int device, unsigned ctas, unsigned capacity) {
+unsigned long long resident_try_acquire(int device, unsigned ctas, unsigned capacity,
+    const int * done) {
   ResGate & g = gate();
   std::lock_guard<std::mutex> lk(g.mu);
-  if (g.next[device] != g.serving[device] ||
-      g.used[device] + std::min(ctas, capacity) > capacity)
-    return false;
-  g.used[device] += std::min(ctas, capacity);
-  return true;
+  ResGate::Device & d = g.devices[device];
+  return d.next != d.serving ? 0 : gate_take(g, d, ctas, capacity, done);
 }
 
-void resident_release(int device, unsigned ctas, unsigned capacity) {
+void resident_release(int device, unsigned long long id) {
   ResGate & g = gate();
   std::lock_guard<std::mutex> lk(g.mu);
-  g.used[device] -= std::min(ctas, capacity);
-  g.cv.notify_all();
+  gate_drop(g, g.devices[device], [&](const ResGate::Held & h) { return h.id == id; });
 }
 
 struct ResidentCg {
@@ -1104,16 +1150,17 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
   }
   g.epoch0 = s->epoch;
   std::memset(s->out_h, 0, sizeof(ResResult));
-  const unsigned units = g.ctas > 1 ? g.ctas : 0;
-  if (units && !resident_acquire(s->a->device, units, s->capacity, cancel_h)) {
-    res->cancelled_waiting = true;
+  unsigned long long held = 0;
+  if (g.ctas > 1 && !(held = resident_acquire(s->a->device, g.ctas, s->capacity, cancel_h,
+                          g.wait_ns, &res->cancelled_waiting))) {
+    res->result.aborted = !res->cancelled_waiting;
     return GOOSEBERRY_SUCCESS;
   }
   void * kargs[] = {&g};
   cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(s->fn),
       dim3(resident_grid(g, s->fault)), dim3(s->threads), kargs, s->smem, stream);
   const cudaError_t e2 = cudaStreamSynchronize(stream);
-  if (units) resident_release(s->a->device, units, s->capacity);
+  resident_release(s->a->device, held);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) {
     s->epoch = 0;

@@ -112,8 +112,8 @@ int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sm
 // loaded at its first use, and what is launched after a load waits until the
 // kernels that run have ended: a request behind a long solve would wait for it.
 int resident_preload();
-// Enqueue a solve.  The caller holds the grid's SMs (resident_acquire) until it
-// has ended, and has cleared words, box, abort flag and r_edge.
+// Enqueue a solve.  The caller holds the grid's SMs (resident_try_acquire) until
+// it has ended, and has cleared words, box, abort flag and r_edge.
 int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream);
 constexpr int kResMaxCtas = 160;  // tagged partials polled, 5 a lane
 
@@ -162,11 +162,15 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
 // one CTA, which waits for nobody.
 bool resident_set_fault(ResidentCg * s, int fault, unsigned limit_ms);
 
-// SMs of a device shared by the grids whose CTAs wait for one another; false
-// if `cancel` (host, may be null) was set before the SMs were free.
-bool resident_acquire(int device, unsigned ctas, unsigned capacity, const int * cancel);
-// The same without waiting: false if the SMs are not free, or others wait.
-bool resident_try_acquire(int device, unsigned ctas, unsigned capacity);
-void resident_release(int device, unsigned ctas, unsigned capacity);
+// SMs of a device shared by the grids whose CTAs wait for one another.  Each
+// returns an id to release them by, or 0.  Waits for them at the head of the
+// queue for limit_ns at most, and not once `cancel` (host, may be null) is set.
+unsigned long long resident_acquire(int device, unsigned ctas, unsigned capacity,
+    const int * cancel, unsigned long long limit_ns, bool * cancelled);
+// Without waiting: 0 if the SMs are not free, or others wait for some.  They are
+// free again when `done` (host, zero now) is set, or when they are released.
+unsigned long long resident_try_acquire(int device, unsigned ctas, unsigned capacity,
+    const int * done);
+void resident_release(int device, unsigned long long id);
 
 }  // namespace gb

@@ -51,6 +51,7 @@
 #include <memory>
 #include <new>
 #include <mutex>
+#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -692,6 +693,7 @@ struct SlotHost {
   int32_t * pats = nullptr;
   uint32_t npat = 0, nnz = 0;
   int stream = -1;
+  unsigned long long held = 0;   // its SMs (resident_try_acquire)
   cudaEvent_t copied = nullptr;  // set at admission, waited for by the first launch
   double tol = 0.0, bnorm = 0.0, rnorm = 0.0;
   size_t iters = 0, rounds = 0;
@@ -753,6 +755,7 @@ struct gb_server {
   std::vector<cudaEvent_t> end;  // per slot: behind its true residual
   int fault = GB_CHIP_FAULT_NONE;  // for tests (gb_server_set_chip_fault)
   unsigned fault_limit_ms = 0;
+  double starved_since = -1.0;  // none of its solves runs and one waits for SMs
 };
 
 namespace gb {
@@ -816,8 +819,7 @@ void destroy_server(gb_server * s) {
       __atomic_store_n(&pinned(*s, k)->cancel, 1, __ATOMIC_RELEASE);
   for (auto & st : s->streams) cudaStreamSynchronize(st);
   for (auto & h : s->slots) {
-    if (h.chip == SlotHost::kRunning)
-      resident_release(s->device, h.shape.args.ctas, chip_capacity(*s));
+    resident_release(s->device, h.held);
     if (h.copied) cudaEventDestroy(h.copied);
   }
   for (auto & st : s->streams) cudaStreamDestroy(st);
@@ -1175,7 +1177,6 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   cudaStream_t st = s.streams[h.stream];
   unsigned char * ctl = s.d_ctl + k * kCtlBytes;
   SrvPinned * pin = pinned(s, k);
-  std::memset(&pin->res, 0, sizeof(pin->res));
   pin->rr_true = 0.0;
   __atomic_store_n(&pin->cancel, 0, __ATOMIC_RELEASE);  // a request to stop belongs to one launch
   GB_CUDA_TRY(cudaStreamWaitEvent(st, h.copied, 0));
@@ -1200,8 +1201,6 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   a.out = &pinned_dev(s, k)->res;
   a.epoch0 = 2;
   a.arrived = reinterpret_cast<unsigned *>(ctl + kCtlFlag + 32);
-  resident_set_waits(&a, s.fault, s.fault_limit_ms);
-  h.shape.fault = s.fault;
   GB_TRY(resident_launch(h.shape, a, st));
   h.chip = SlotHost::kRunning;
   return GOOSEBERRY_SUCCESS;
@@ -1211,6 +1210,22 @@ bool chip_done(gb_server & s, uint32_t k) {
   return __atomic_load_n(&pinned(s, k)->res.done, __ATOMIC_ACQUIRE) != 0;
 }
 
+// Slot k's request goes to the batch, from the start.
+int to_batch(gb_server & s, uint32_t k) {
+  SlotHost & h = s.slots[k];
+  if (h.stream >= 0) s.free_streams.push_back(h.stream);
+  h.stream = -1;
+  SrvSlot S = h.dev;
+  if (s.mixed && h.nnz)
+    GB_TRY(launch_round_f32(S.val64, const_cast<float *>(S.val32), h.nnz, s.stream));
+  cudaEventDestroy(h.copied);
+  h.copied = nullptr;
+  h.chip = SlotHost::kBatch;
+  s.h_slots[k] = S;
+  s.dirty = true;
+  return GOOSEBERRY_SUCCESS;
+}
+
 // Take slot k's ended solve: finished, or back to the batch (a wait inside it
 // was given up); in mixed mode its true residual is formed first.
 int collect_on_chip(gb_server & s, uint32_t k) {
@@ -1218,20 +1233,11 @@ int collect_on_chip(gb_server & s, uint32_t k) {
   const SrvPinned & pin = *pinned(s, k);
   s.stats.gpu_ms += (pin.res.t1 - pin.res.t0) * 1e-6 * h.shape.args.ctas /  // its share of the
                     std::max(1, s.sm_count);                                // device
-  resident_release(s.device, h.shape.args.ctas, chip_capacity(s));
+  resident_release(s.device, h.held);
+  h.held = 0;
   if (pin.res.aborted) {
     GB_CUDA_TRY(cudaStreamSynchronize(s.streams[h.stream]));
-    s.free_streams.push_back(h.stream);
-    h.stream = -1;
-    SrvSlot S = h.dev;
-    if (s.mixed && h.nnz)
-      GB_TRY(launch_round_f32(S.val64, const_cast<float *>(S.val32), h.nnz, s.stream));
-    cudaEventDestroy(h.copied);
-    h.copied = nullptr;
-    h.chip = SlotHost::kBatch;
-    s.h_slots[k] = S;
-    s.dirty = true;
-    return GOOSEBERRY_SUCCESS;
+    return to_batch(s, k);
   }
   h.iters += pin.res.iter;
   h.status = pin.res.status;
@@ -1617,17 +1623,37 @@ int step(gb_server & s, size_t * active, size_t * queued) {
                                                     : p < q;
   });
   for (uint32_t k : wait) {
-    const unsigned ctas = s.slots[k].shape.args.ctas;
-    if (!resident_try_acquire(s.device, ctas, chip_capacity(s))) {
-      if (now_s(s) - s.slots[k].t_admit > 0.02) break;
+    SlotHost & h = s.slots[k];
+    std::memset(&pinned(s, k)->res, 0, sizeof(ResResult));
+    resident_set_waits(&h.shape.args, s.fault, s.fault_limit_ms);
+    h.shape.fault = s.fault;
+    h.held = resident_try_acquire(s.device, h.shape.args.ctas, chip_capacity(s),
+        &pinned(s, k)->res.done);
+    if (!h.held) {
+      if (now_s(s) - h.t_admit > 0.02) break;
       continue;
     }
     const int rc = launch_on_chip(s, k);
     if (rc != GOOSEBERRY_SUCCESS) {
-      resident_release(s.device, ctas, chip_capacity(s));
+      resident_release(s.device, h.held);
+      h.held = 0;
       return rc;
     }
     launched = true;
+  }
+  // nothing of this server runs on the chip, and others have not left the SMs to
+  // the longest waiting request for as long as any wait may take: the batch
+  bool on_chip = false;
+  for (const auto & h : s.slots)
+    on_chip |= h.used && (h.chip == SlotHost::kRunning || h.chip == SlotHost::kChecking);
+  if (wait.empty() || on_chip) {
+    s.starved_since = -1.0;
+  } else if (s.starved_since < 0.0) {
+    s.starved_since = now_s(s);
+  } else if (now_s(s) - s.starved_since > 1e-9 * s.slots[wait[0]].shape.args.wait_ns) {
+    GB_TRY(to_batch(s, wait[0]));
+    s.starved_since = -1.0;
+    moved = true;
   }
   // 3. rebuild the tile list and upload the slot table
   size_t nact = 0;
@@ -1661,7 +1687,11 @@ int step(gb_server & s, size_t * active, size_t * queued) {
   if (launched && !nbatch) s.stats.steps += 1;
   // with nothing to do but wait for solves on the chip, wait for one (at most
   // a millisecond, so that a caller's submissions and cancels get their turn)
-  if (running && !nbatch && !moved && !launched) {
+  if (!running && !wait.empty() && !nbatch && !moved) {
+    std::this_thread::sleep_for(std::chrono::microseconds(200));  // others hold the SMs
+    s.stats.wait_ms += 0.2;
+    waited += 0.2;
+  } else if (running && !nbatch && !moved && !launched) {
     const auto w0 = std::chrono::steady_clock::now();
     bool ended = false;
     while (!ended) {
