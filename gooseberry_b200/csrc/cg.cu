@@ -1578,7 +1578,7 @@ int solve_resident(gb_cg * s, const double * b, double * x, double tol, int tol_
       aborted = r.aborted != 0;
       if (aborted) return GOOSEBERRY_SUCCESS;
       status = out.cancelled_waiting ? GB_CG_CANCELLED : r.status;
-      launches += out.cancelled_waiting ? 0 : 1;
+      launches += out.launches;
       const unsigned g = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(
           (s->n + kVecBlock - 1) / kVecBlock, static_cast<size_t>(s->a->sm_count) * 4)));
       if (out.cancelled_waiting) {
@@ -1905,7 +1905,7 @@ int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned limit_ms) {
 
 int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms) {
   GB_CHECK_INPUT(s != nullptr, "solver is NULL");
-  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_LATE, "unknown fault %d",
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_SHORT, "unknown fault %d",
       fault);
   GB_CHECK_INPUT(s->resident && gb::resident_set_fault(s->resident, fault, limit_ms),
       "the fault applies to solves on the chip by more than one CTA");

@@ -51,6 +51,12 @@
 // neighbours' r take behind it), r 570, two divisions 600.  Small systems wait
 // for the two exchanges, which cost what L2 does: 2,100 clocks each.
 //
+// A launch runs for as many iterations as take about kResSliceNs, writes r and p
+// beside x and ends, so that other streams' kernels, which find no room on SMs
+// held so, get their turn; the next launch goes on with the same bits.  (A clock
+// read by the CTAs and a request to pause sent with the sums cost 2-5% of every
+// iteration; the count costs nothing, as the limit is checked anyway.)
+//
 // A wait that lasts longer than a limit raises the abort flag; every CTA
 // leaves, and the host runs the solve on the graph path instead.
 #include <algorithm>
@@ -80,6 +86,9 @@ constexpr int kResThreadsWide = 384, kResRowsWide = 19;
 // rows: 2.68 us an iteration, 3.36 over four CTAs; 2,304 rows: 3.41 and 3.39).
 constexpr uint32_t kResOneCta = 2048;
 constexpr unsigned long long kResWaitNs = 2000000000ull;
+// A launch's time: how often what waits for SMs (other solves, other streams'
+// kernels) gets its turn.  A launch more costs 22 us at 400^2, 31 us at 1024^2.
+constexpr double kResSliceNs = 1e7;
 
 // How a CTA finds its matrix rows.
 enum ResSource {
@@ -185,8 +194,7 @@ __device__ __forceinline__ double warp_allsum(double v) {
 struct ResShared {
   double red[32];
   double total;
-  int bad;         // a wait for a neighbour's r was given up
-  int leave;       // that, or a wait of this all-reduce's: what all threads go by
+  int bad;         // a wait in this CTA was given up
   int cancel;      // the host asked to stop (CTA 0's view, as of this all-reduce)
   int cancel_req;  // CTA 0: what it will send
   double bnorm, tol, rr_far;
@@ -201,8 +209,8 @@ struct ResSums {
 
 // Every CTA's `v` by tagged messages, added in CTA order: lane l adds those of
 // CTAs l, l + 32, ..., then the warp tree.  All lanes of warp 0 call it.
-__device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResSums & st,
-    uint32_t epoch, double v, int * cancel, int * bad) {
+__device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResShared & sh, ResSums & st,
+    uint32_t epoch, double v, int * cancel) {
   const int lane = threadIdx.x & 31;
   ulonglong2 * const box = a.box + (st.tagged++ & 1) * a.ctas;
   const uint32_t tag = epoch << 1;
@@ -215,7 +223,7 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResSums & st
     ulonglong2 m = tagged_load(box + c);
     while (!tag_is(make_ulonglong2(m.x & kNoCancel, m.y & kNoCancel), tag)) {
       if (res_give_up(a, ++polls, &t0)) {
-        *bad = 1;
+        sh.bad = 1;
         break;
       }
       m = tagged_load(box + c);
@@ -224,7 +232,6 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResSums & st
     if (c == 0) *cancel = static_cast<int>((m.x >> 32) & 1u);
   }
   *cancel = __shfl_sync(0xffffffffu, *cancel, 0);
-  *bad = __any_sync(0xffffffffu, *bad);
   return warp_allsum(acc);
 }
 
@@ -237,8 +244,8 @@ __device__ __forceinline__ double res_sum_tagged(const ResArgs & a, ResSums & st
 // fit or the sum is so much smaller than `prev` that the cut-off bits
 // (2^(E - 131) a CTA) would show in its 53.
 template <class S>
-__device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResSums & st, double v,
-    double prev, int * cancel, int * bad, double * total, S && sent) {
+__device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResShared & sh, ResSums & st,
+    double v, double prev, int * cancel, double * total, S && sent) {
   const int lane = threadIdx.x & 31;
   const int e = ((__double2hiint(prev) >> 20) & 0x7ff) - 1023 + 40;
   const bool odd = st.fixed++ & 1;
@@ -270,7 +277,7 @@ __device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResSums & st, d
     const bool all = lane >= 3 || static_cast<uint32_t>((cur - seen) >> 56) == a.ctas;
     if (__all_sync(0xffffffffu, all)) break;
     if (__any_sync(0xffffffffu, res_give_up(a, polls, &t0))) {
-      *bad = 1;
+      sh.bad = 1;
       break;
     }
   }
@@ -297,9 +304,9 @@ __device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResSums & st, d
 // Sum of every CTA's `local` (over its threads), the same bits in every CTA.
 // `prev`: a sum of about this size, the same in every CTA (0: unknown).  Warps
 // 1.. run `hidden` while warp 0 exchanges the sums, and warp 0
-// runs `sent` between its send and its wait.  Returns false, in every thread of
-// the CTA alike, when a wait was given up before the sum was complete (a wait
-// of `hidden` that is given up later is told by the next all-reduce).
+// runs `sent` between its send and its wait.  Returns false when a wait was
+// given up, in every thread of the CTA alike: sh.bad is written between the two
+// barriers here, and elsewhere only behind a barrier that follows.
 template <int T, class F, class S>
 __device__ __forceinline__ bool res_allreduce(const ResArgs & a, ResShared & sh, ResSums & st,
     uint32_t & epoch, double local, double prev, F && hidden, S && sent, double * total) {
@@ -310,28 +317,27 @@ __device__ __forceinline__ bool res_allreduce(const ResArgs & a, ResShared & sh,
   if (warp == 0) {
     const double v = warp_allsum(lane < T / 32 ? sh.red[lane] : 0.0);
     double sum = v;
-    int cancel = sh.cancel_req, bad = sh.bad;
+    int cancel = sh.cancel_req;
     if (a.ctas > 1) {
       // (the bounds keep the fixed point's unit and the sum normal)
       const bool known = prev > 0x1p-960 && prev < INFINITY;
       const int asked = cancel;
       if (!known) sent();
-      if (!known || !res_sum_fixed(a, st, v, prev, &cancel, &bad, &sum, sent)) {
+      if (!known || !res_sum_fixed(a, sh, st, v, prev, &cancel, &sum, sent)) {
         cancel = asked;
-        sum = res_sum_tagged(a, st, epoch, v, &cancel, &bad);
+        sum = res_sum_tagged(a, sh, st, epoch, v, &cancel);
       }
     }
     if (lane == 0) {
       sh.total = sum;
       sh.cancel = cancel;
-      sh.leave = bad;
     }
   } else {
     hidden();
   }
   __syncthreads();
   *total = sh.total;
-  return sh.leave == 0;
+  return sh.bad == 0;
 }
 
 // One thread's cached view of a row pattern (and, for RES_CLASS, its values):
@@ -463,7 +469,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
   // hoisted out of the solve's loop they would take the registers that hold r.
   const auto reform = [&] { asm volatile("" : "+r"(lo), "+r"(nloc), "+r"(H), "+r"(tid)); };
 
-  // ---- the CTA's matrix rows, x = 0, r = b, p = 0 ----
+  // ---- the CTA's matrix rows; x = 0, r = b, p = 0, or where the last launch ended ----
   if constexpr (SRC != RES_CSR) {
     unsigned char * const t = smem + L.table;
     const uint32_t tw = static_cast<uint32_t>(
@@ -495,7 +501,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
       }
     }
   }
-  if (a.arrived && blockIdx.x == 0 && tid == 0) a.out->t0 = res_ns();
+  if (blockIdx.x == 0 && tid == 0) a.out->t0 = res_ns();
   if (tid == 0) {
     sh.bad = 0;
     sh.cancel = 0;
@@ -515,13 +521,16 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     r[k] = 0.0;
     if (k * T < nloc) aps[i] = 0.0;  // rows past the block's end keep r = Ap = 0
     if (i < nloc) {
-      r[k] = a.b[lo + i];
-      if (a.at.x) xs[i] = 0.0;
-      else a.x[lo + i] = 0.0;
+      r[k] = a.resume ? a.r_save[lo + i] : a.b[lo + i];
+      if (a.at.x) xs[i] = a.resume ? a.x[lo + i] : 0.0;
+      else if (!a.resume) a.x[lo + i] = 0.0;
       acc = fma(r[k], r[k], acc);
     }
   }
-  for (uint32_t i = tid; i < nloc + 2 * H; i += T) pw[i] = 0.0;
+  for (uint32_t i = tid; i < nloc + 2 * H; i += T) {
+    const uint32_t g = lo - H + i;  // wraps to >= n outside the matrix
+    pw[i] = a.resume && g < a.n ? a.p_save[g] : 0.0;
+  }
 
   // ---- the neighbours' r ----
   // Halo entry j: the H rows below the block, then the H rows above it.  With
@@ -582,8 +591,13 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     publish();
     prefetch_halo();
   }, publish, &rr);
+  if (a.resume) {
+    rr = a.rr0;
+    pap = a.pap0;
+    beta = a.beta0;
+  }
   if (tid == 0) {
-    sh.bnorm = sqrt(rr);
+    sh.bnorm = a.resume ? a.bnorm0 : sqrt(rr);
     const double tol = a.tol_relative ? a.tol * sh.bnorm : a.tol;
     sh.tol = tol;
     // r.r above this means ||r|| > tol without taking the root (infinite where
@@ -591,7 +605,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     sh.rr_far = tol > 1e-140 ? tol * tol * (1.0 + 1e-14) : INFINITY;
   }
   __syncthreads();
-  unsigned long long it = 0, t_a = 0, t_b = 0;  // t_a, t_b: ns in A and B (a.timed)
+  unsigned long long it = a.resume ? a.it0 : 0, t_a = 0, t_b = 0;  // t_a, t_b: ns in A and B (a.timed)
   int status = GB_CG_MAXITER;
   bool running = ok;
   if (rr == 0.0) {
@@ -611,6 +625,7 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
         pw[win] = fma(beta, pw[win], rh[j]);
       }
     } else {
+      __syncthreads();  // all have read sh.bad
       halo_fetch(tid, T, [&](uint32_t j, double v) {
         const uint32_t win = halo_win(j);
         pw[win] = fma(beta, pw[win], v);
@@ -743,13 +758,24 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     rr = rr_new;
   }
   __syncthreads();
+  const bool more = a.more && status == GB_CG_MAXITER;
+  if (ok && more) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (k * T + tid < nloc) a.r_save[lo + k * T + tid] = r[k];
+    for (uint32_t i = tid; i < nloc; i += T) a.p_save[lo + i] = po[i];
+  }
   if (ok && a.at.x)
     for (uint32_t i = tid; i < nloc; i += T) a.x[lo + i] = xs[i];
   if (blockIdx.x == 0 && tid == 0) {
-    a.out->status = status;
+    a.out->status = more ? kResPaused : status;
     a.out->iter = it;
     a.out->rr = rr;
     a.out->bnorm = sh.bnorm;
+    a.out->pap = pap;
+    a.out->beta = beta;
+    a.out->ran = it - (a.resume ? a.it0 : 0);
+    a.out->t1 = res_ns();
     a.out->epoch = epoch;
     a.out->ns_a = t_a;
     a.out->ns_b = t_b;
@@ -905,6 +931,7 @@ struct ResidentCg {
   unsigned long long * words = nullptr;  // [32]
   ulonglong2 * box = nullptr;
   size_t box_bytes = 0;      // the tagged partials and, behind them, the abort flag
+  double * save = nullptr;   // [2][n] r and p of a solve between two launches
   ResResult * out_h = nullptr;
   ResResult * out_d = nullptr;
   RowClasses classes;
@@ -923,6 +950,7 @@ void resident_destroy(ResidentCg * s) {
   dev_free(s->r_edge);
   dev_free(s->words);
   dev_free(s->box);
+  dev_free(s->save);
   pinned_slot_free(s->out_h);
   free_row_classes(s->classes);
   delete s;
@@ -1108,8 +1136,41 @@ int resident_create(const gb_csr & a, const ResidentIn & in, double * x, Residen
   g.box = s->box;
   g.abort_flag = reinterpret_cast<int *>(reinterpret_cast<char *>(s->box) + s->box_bytes);
   g.out = s->out_d;
+  if (dev_alloc(&s->save, 2 * static_cast<size_t>(n) * sizeof(double)) == GOOSEBERRY_SUCCESS) {
+    g.r_save = s->save;
+    g.p_save = s->save + n;
+  } else {
+    cudaGetLastError();  // no memory to pause with: one launch
+    s->save = nullptr;
+  }
   *out = s;
   return GOOSEBERRY_SUCCESS;
+}
+
+void resident_slice(ResArgs * g, unsigned long long niter, int fault, const ResResult * last) {
+  g->niter = niter;
+  g->more = 0;
+  if (!g->p_save) return;  // no memory to go on from: one launch
+  // The first launch's iterations by the rows of a CTA, estimated long (3 us and
+  // 0.8 to 1.6 ns a row, see above); the others' as long as the last one's.
+  double n = kResSliceNs / (4000.0 + 1.6 * g->rows);
+  if (last)
+    n = static_cast<double>(last->ran) * kResSliceNs /
+        std::max<double>(1.0, static_cast<double>(last->t1 - last->t0));
+  const unsigned long long from = last ? last->iter : 0;
+  const unsigned long long upto = from + (fault == GB_CHIP_FAULT_SHORT
+      ? 64 : static_cast<unsigned long long>(std::max(n, 64.0)));
+  if (!niter || upto < niter) {
+    g->niter = upto;
+    g->more = 1;
+  }
+  if (!last) return;
+  g->resume = 1;
+  g->it0 = last->iter;
+  g->rr0 = last->rr;
+  g->pap0 = last->pap;
+  g->beta0 = last->beta;
+  g->bnorm0 = last->bnorm;
 }
 
 void resident_set_waits(ResArgs * g, int fault, unsigned limit_ms) {
@@ -1138,38 +1199,45 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
   g.hist_len = hist_len;
   g.cancel = cancel_d;
   *res = ResOutcome{};
-  // Tags of one solve must not meet those that earlier solves left in memory:
-  // the count goes on from solve to solve, and starts over, with cleared
-  // memory, before it could wrap (a tag is the count's low 31 bits).
-  if (s->epoch == 0 || s->epoch > (1u << 29)) {
-    GB_CUDA_TRY(cudaMemsetAsync(s->words, 0, 32 * sizeof(unsigned long long), stream));
-    GB_CUDA_TRY(cudaMemsetAsync(s->box, 0, s->box_bytes + 16, stream));
-    GB_CUDA_TRY(cudaMemsetAsync(s->r_edge, 0, static_cast<size_t>(g.n) * sizeof(ulonglong2),
-        stream));
-    s->epoch = 2;
-  }
-  g.epoch0 = s->epoch;
-  std::memset(s->out_h, 0, sizeof(ResResult));
-  unsigned long long held = 0;
-  if (g.ctas > 1 && !(held = resident_acquire(s->a->device, g.ctas, s->capacity, cancel_h,
-                          g.wait_ns, &res->cancelled_waiting))) {
-    res->result.aborted = !res->cancelled_waiting;
-    return GOOSEBERRY_SUCCESS;
-  }
-  void * kargs[] = {&g};
-  cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(s->fn),
-      dim3(resident_grid(g, s->fault)), dim3(s->threads), kargs, s->smem, stream);
-  const cudaError_t e2 = cudaStreamSynchronize(stream);
-  resident_release(s->a->device, held);
-  if (e == cudaSuccess) e = e2;
-  if (e != cudaSuccess) {
-    s->epoch = 0;
-    set_error("CG solve failed: %s", cudaGetErrorString(e));
-    return GOOSEBERRY_ERROR_UNKNOWN;
-  }
-  res->result = *s->out_h;
-  // an abandoned solve leaves the CTAs at different counts
-  s->epoch = s->out_h->aborted ? 0 : s->out_h->epoch;
+  do {
+    if (!timed) resident_slice(&g, niter, s->fault, res->launches ? &res->result : nullptr);
+    // Tags of one launch must not meet those that earlier ones left in memory:
+    // the count goes on from launch to launch, and starts over, with cleared
+    // memory, before it could wrap (a tag is the count's low 31 bits).
+    if (s->epoch == 0 || s->epoch > (1u << 29)) {
+      GB_CUDA_TRY(cudaMemsetAsync(s->words, 0, 32 * sizeof(unsigned long long), stream));
+      GB_CUDA_TRY(cudaMemsetAsync(s->box, 0, s->box_bytes + 16, stream));
+      GB_CUDA_TRY(cudaMemsetAsync(s->r_edge, 0, static_cast<size_t>(g.n) * sizeof(ulonglong2),
+          stream));
+      s->epoch = 2;
+    }
+    g.epoch0 = s->epoch;
+    unsigned long long held = 0;
+    bool cancelled = false;
+    if (g.ctas > 1 && !(held = resident_acquire(s->a->device, g.ctas, s->capacity, cancel_h,
+                            g.wait_ns, &cancelled))) {
+      if (!cancelled) res->result.aborted = 1;
+      else if (g.resume) res->result.status = GB_CG_CANCELLED;  // x is that of the last launch
+      else res->cancelled_waiting = true;
+      return GOOSEBERRY_SUCCESS;
+    }
+    std::memset(s->out_h, 0, sizeof(ResResult));
+    void * kargs[] = {&g};
+    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(s->fn),
+        dim3(resident_grid(g, s->fault)), dim3(s->threads), kargs, s->smem, stream);
+    const cudaError_t e2 = cudaStreamSynchronize(stream);
+    resident_release(s->a->device, held);
+    if (e == cudaSuccess) e = e2;
+    if (e != cudaSuccess) {
+      s->epoch = 0;
+      set_error("CG solve failed: %s", cudaGetErrorString(e));
+      return GOOSEBERRY_ERROR_UNKNOWN;
+    }
+    res->result = *s->out_h;
+    ++res->launches;
+    // an abandoned solve leaves the CTAs at different counts
+    s->epoch = s->out_h->aborted ? 0 : s->out_h->epoch;
+  } while (!res->result.aborted && res->result.status == kResPaused);
   return GOOSEBERRY_SUCCESS;
 }
 

@@ -47,12 +47,17 @@ struct ResResult {
   int status;
   int aborted;  // some CTA gave up waiting
   unsigned long long iter;
+  unsigned long long ran;  // iterations of this launch
   double rr, bnorm;
+  double pap, beta;  // of the last iteration, for a solve that goes on
   unsigned epoch;  // all-reduces so far
   unsigned long long ns_a, ns_b;  // time in the two phases (a timed solve)
-  unsigned long long t0, t1;      // begin and end (with ResArgs::arrived)
+  unsigned long long t0, t1;      // begin and end
   int done;                       // written last (with ResArgs::arrived)
 };
+
+// `status` of a launch that ended before its solve (ResArgs::more).
+constexpr int kResPaused = 100;
 
 // ---- the solve kernel's arguments ------------------------------------------------
 // What has a place in shared memory besides p, Ap, the tables and the row bytes.
@@ -88,6 +93,13 @@ struct ResArgs {
   uint32_t epoch0;
   double tol;
   int timed;                      // report the phases' times
+  // With `more` the launch's niter is not the solve's: it leaves r and p in r_save
+  // and p_save [n].  One that goes on takes them, x and the scalars below.
+  double * r_save;
+  double * p_save;
+  int more, resume;
+  unsigned long long it0;
+  double rr0, pap0, beta0, bnorm0;
   unsigned long long wait_ns;     // a wait that lasts longer is given up
   unsigned long long late_ns;     // for tests: CTA 0 is that late after iteration 64
   unsigned * arrived;             // may be null; 0 before: count the CTAs out, so that the last
@@ -104,6 +116,9 @@ struct ResShape {
   int threads = 0;
   int fault = GB_CHIP_FAULT_NONE;  // for tests
 };
+// The niter of a solve's next launch, after `last` (null: the first); with
+// p_save null there is only one.
+void resident_slice(ResArgs * g, unsigned long long niter, int fault, const ResResult * last);
 // Sets the limit of a solve's waits (0: the usual one) and, for tests, a fault.
 void resident_set_waits(ResArgs * g, int fault, unsigned limit_ms);
 int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,
@@ -127,6 +142,7 @@ int preload_true_residual();  // loads the two kernels above
 
 struct ResOutcome {
   ResResult result{};
+  unsigned launches = 0;
   bool cancelled_waiting = false;  // cancelled before it got its SMs
 };
 

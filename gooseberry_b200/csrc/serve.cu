@@ -688,6 +688,12 @@ struct SlotHost {
   ResShape shape;
   SrvSlot dev{};                 // its device arrays (and the batch's, should it fall back)
   double * d = nullptr;          // refinement's correction (mixed)
+  // r and p between two launches of the solve, and p between two of a correction;
+  // p_save is null where the request's arrays have no room (one launch then)
+  double * r_save = nullptr;
+  double * p_save[2] = {nullptr, nullptr};
+  bool resume = false;           // the next launch goes on where `paused` ended
+  ResResult paused{};
   ulonglong2 * r_edge = nullptr;
   uint8_t * codes = nullptr;
   int32_t * pats = nullptr;
@@ -1113,6 +1119,23 @@ int admit(gb_server & s, Request & q, uint32_t k) {
     }
     h.pats = reinterpret_cast<int32_t *>(more);
     h.codes = reinterpret_cast<uint8_t *>(more + align256(32ull * q.npat));
+    // r and p of a paused solve: over the correction and its right-hand side,
+    // which are not in use yet (mixed), or behind the row bytes; a correction's
+    // r over its right-hand side, which is read at its start alone
+    double * behind = reinterpret_cast<double *>(more + align256(32ull * q.npat) +
+                                                 align256(q.n));
+    const size_t dn = align256(8ull * q.n);
+    const char * end = s.mixed ? reinterpret_cast<char *>(v32) + align256(4ull * q.nnz)
+                               : static_cast<char *>(y) + 5 * dn;
+    const size_t room = static_cast<size_t>(end - reinterpret_cast<char *>(behind));
+    if (s.mixed) {
+      h.r_save = x1;
+      h.p_save[0] = h.d;
+      h.p_save[1] = room >= dn ? behind : nullptr;
+    } else {
+      h.r_save = behind;
+      h.p_save[0] = room >= 2 * dn ? behind + dn / 8 : nullptr;
+    }
     GB_CUDA_TRY(cudaMemcpyAsync(h.pats, q.pats, 32ull * q.npat, cudaMemcpyHostToDevice, s.stream));
     GB_CUDA_TRY(cudaMemcpyAsync(h.codes, q.codes, q.n, cudaMemcpyHostToDevice, s.stream));
     GB_CUDA_TRY(cudaEventCreateWithFlags(&h.copied, cudaEventDisableTiming));
@@ -1185,7 +1208,6 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   ResArgs a = h.shape.args;
   a.tol_relative = h.rounds ? 0 : 1;
   a.tol = h.rounds ? h.tol : S.tol_rel;
-  a.niter = S.niter - h.iters;
   a.row_code = h.codes;
   a.pat_off = h.pats;
   a.rowptr = S.rowptr;
@@ -1194,6 +1216,9 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   a.b = h.rounds ? S.x1 : S.b;
   a.x = h.rounds ? h.d : S.x0;
   a.r_edge = h.r_edge;
+  a.r_save = h.r_save;
+  a.p_save = h.p_save[h.rounds ? 1 : 0];
+  resident_slice(&a, S.niter - h.iters, s.fault, h.resume ? &h.paused : nullptr);
   a.words = reinterpret_cast<unsigned long long *>(ctl);
   a.box = reinterpret_cast<ulonglong2 *>(ctl + kCtlBox);
   a.abort_flag = reinterpret_cast<int *>(ctl + kCtlFlag);
@@ -1226,7 +1251,8 @@ int to_batch(gb_server & s, uint32_t k) {
   return GOOSEBERRY_SUCCESS;
 }
 
-// Take slot k's ended solve: finished, or back to the batch (a wait inside it
+// Take slot k's ended launch: the solve goes on with another one, is finished,
+// or goes back to the batch (a wait inside it
 // was given up); in mixed mode its true residual is formed first.
 int collect_on_chip(gb_server & s, uint32_t k) {
   SlotHost & h = s.slots[k];
@@ -1239,8 +1265,16 @@ int collect_on_chip(gb_server & s, uint32_t k) {
     GB_CUDA_TRY(cudaStreamSynchronize(s.streams[h.stream]));
     return to_batch(s, k);
   }
+  h.resume = pin.res.status == kResPaused && !h.cancel;
+  if (h.resume) {
+    h.paused = pin.res;
+    s.free_streams.push_back(h.stream);
+    h.stream = -1;
+    h.chip = SlotHost::kWaiting;
+    return GOOSEBERRY_SUCCESS;
+  }
   h.iters += pin.res.iter;
-  h.status = pin.res.status;
+  h.status = pin.res.status == kResPaused ? static_cast<int>(GB_CG_CANCELLED) : pin.res.status;
   h.rnorm = std::sqrt(pin.res.rr);
   if (h.rounds == 0) {
     h.bnorm = pin.res.bnorm;
@@ -1570,10 +1604,10 @@ int step(gb_server & s, size_t * active, size_t * queued) {
       res.bnorm = S.bnorm;
       res.status = S.done ? S.status : GB_CG_CANCELLED;
     } else {
-      res.iterations = h.iters;
+      res.iterations = h.iters + (h.resume ? h.paused.iter : 0);
       res.refinements = h.rounds;
-      res.rnorm = h.rnorm;
-      res.bnorm = h.bnorm;
+      res.rnorm = h.resume ? std::sqrt(h.paused.rr) : h.rnorm;
+      res.bnorm = h.resume && h.rounds == 0 ? h.paused.bnorm : h.bnorm;
       res.status = h.chip == SlotHost::kFinished ? h.status : GB_CG_CANCELLED;
       if (h.copied) {
         GB_CUDA_TRY(cudaEventSynchronize(h.copied));  // (cancelled before it was launched)
@@ -1795,7 +1829,7 @@ int gb_server_cancel(gb_server_t * s, uint64_t id) {
 
 int gb_server_set_chip_fault(gb_server_t * s, int fault, unsigned limit_ms) {
   GB_CHECK_INPUT(s != nullptr, "server is NULL");
-  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_LATE, "unknown fault %d",
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_SHORT, "unknown fault %d",
       fault);
   s->fault = fault;
   s->fault_limit_ms = limit_ms;

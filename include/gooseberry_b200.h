@@ -264,9 +264,11 @@ typedef enum gb_cg_mode {
  * distinct column-offset patterns (stencils) whose vectors fit the SMs'
  * shared memory (up to about 1.08 million rows on 148 SMs, fewer with a wide
  * band) is solved in one cooperative launch with the vectors on the chip.
- * Such solves of one process share a device's SMs: each holds as many as it
- * has CTAs until it ends, and waits for them in order of arrival.  Should a
- * wait inside a solve exceed 2 s (another program holds SMs), the solve is run
+ * Such solves of one process share a device's SMs: each launch holds as many as
+ * it has CTAs, and waits for them in order of arrival.  A solve of more than
+ * about 10 ms takes several launches, with the same results, so that other
+ * solves and other streams' kernels get their turn.  Should a wait for SMs, or
+ * inside a solve, exceed 2 s (another program holds them), the solve is run
  * again by the graph-replayed kernels. */
 
 /* OR-ed into the mode of gb_cg_create: run the whole solve as ONE persistent
@@ -352,13 +354,15 @@ GOOSEBERRY_API int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned l
  * late after iteration 64 by twice the wait limit (LATE).  The other CTAs give
  * up when the limit is over, raise the abort flag and leave (as a late one then
  * does), and the call runs the solve by the graph-replayed kernels and returns
- * their result.  `limit_ms` sets the limit (0: 2000).  Nothing waits without
+ * their result.  With SHORT every launch of a solve ends at its first check of
+ * the time, some 64 iterations, and the next goes on.  `limit_ms` sets the limit (0: 2000).  Nothing waits without
  * one, so the device stays usable.  Refused for a solver that does not solve on
  * the chip, or that does on one CTA.  No reference counterpart. */
 typedef enum gb_chip_fault {
   GB_CHIP_FAULT_NONE = 0,
   GB_CHIP_FAULT_MISSING = 1,
-  GB_CHIP_FAULT_LATE = 2
+  GB_CHIP_FAULT_LATE = 2,
+  GB_CHIP_FAULT_SHORT = 3
 } gb_chip_fault_t;
 GOOSEBERRY_API int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms);
 
