@@ -86,9 +86,6 @@ constexpr int kResThreadsWide = 384, kResRowsWide = 19;
 // rows: 2.68 us an iteration, 3.36 over four CTAs; 2,304 rows: 3.41 and 3.39).
 constexpr uint32_t kResOneCta = 2048;
 constexpr unsigned long long kResWaitNs = 2000000000ull;
-// A launch's time: how often what waits for SMs (other solves, other streams'
-// kernels) gets its turn.  A launch more costs 22 us at 400^2, 31 us at 1024^2.
-constexpr double kResSliceNs = 1e7;
 
 // How a CTA finds its matrix rows.
 enum ResSource {
@@ -1147,15 +1144,16 @@ int resident_create(const gb_csr & a, const ResidentIn & in, double * x, Residen
   return GOOSEBERRY_SUCCESS;
 }
 
-void resident_slice(ResArgs * g, unsigned long long niter, int fault, const ResResult * last) {
+void resident_slice(ResArgs * g, unsigned long long niter, int fault, double ns,
+    const ResResult * last) {
   g->niter = niter;
   g->more = 0;
   if (!g->p_save) return;  // no memory to go on from: one launch
   // The first launch's iterations by the rows of a CTA, estimated long (3 us and
   // 0.8 to 1.6 ns a row, see above); the others' as long as the last one's.
-  double n = kResSliceNs / (4000.0 + 1.6 * g->rows);
+  double n = ns / (4000.0 + 1.6 * g->rows);
   if (last)
-    n = static_cast<double>(last->ran) * kResSliceNs /
+    n = static_cast<double>(last->ran) * ns /
         std::max<double>(1.0, static_cast<double>(last->t1 - last->t0));
   const unsigned long long from = last ? last->iter : 0;
   const unsigned long long upto = from + (fault == GB_CHIP_FAULT_SHORT
@@ -1200,7 +1198,8 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
   g.cancel = cancel_d;
   *res = ResOutcome{};
   do {
-    if (!timed) resident_slice(&g, niter, s->fault, res->launches ? &res->result : nullptr);
+    if (!timed) resident_slice(&g, niter, s->fault, kResSliceNs,
+                    res->launches ? &res->result : nullptr);
     // Tags of one launch must not meet those that earlier ones left in memory:
     // the count goes on from launch to launch, and starts over, with cleared
     // memory, before it could wrap (a tag is the count's low 31 bits).

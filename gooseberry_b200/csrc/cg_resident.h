@@ -116,9 +116,13 @@ struct ResShape {
   int threads = 0;
   int fault = GB_CHIP_FAULT_NONE;  // for tests
 };
-// The niter of a solve's next launch, after `last` (null: the first); with
-// p_save null there is only one.
-void resident_slice(ResArgs * g, unsigned long long niter, int fault, const ResResult * last);
+// A launch's time: how often what waits for SMs (other solves, other streams'
+// kernels) gets its turn.  A launch more costs 22 us at 400^2, 31 us at 1024^2.
+constexpr double kResSliceNs = 1e7;
+// The niter of a solve's next launch, of about `ns`, after `last` (null: the
+// first); with p_save null there is only one.
+void resident_slice(ResArgs * g, unsigned long long niter, int fault, double ns,
+    const ResResult * last);
 // Sets the limit of a solve's waits (0: the usual one) and, for tests, a fault.
 void resident_set_waits(ResArgs * g, int fault, unsigned limit_ms);
 int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sms, uint32_t want,

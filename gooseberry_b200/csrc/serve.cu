@@ -757,6 +757,7 @@ struct gb_server {
   unsigned char * h_pin = nullptr;      // [max_slots] pinned blocks
   unsigned char * d_pin = nullptr;      // their device address
   std::vector<cudaStream_t> streams;    // made as they are needed
+  cudaStream_t copies = nullptr;        // solutions of solves on the chip
   std::vector<int> free_streams;
   std::vector<cudaEvent_t> end;  // per slot: behind its true residual
   int fault = GB_CHIP_FAULT_NONE;  // for tests (gb_server_set_chip_fault)
@@ -829,6 +830,7 @@ void destroy_server(gb_server * s) {
     if (h.copied) cudaEventDestroy(h.copied);
   }
   for (auto & st : s->streams) cudaStreamDestroy(st);
+  if (s->copies) cudaStreamDestroy(s->copies);
   for (auto & e : s->end)
     if (e) cudaEventDestroy(e);
   cudaFree(s->d_ctl);
@@ -908,6 +910,7 @@ int create_server(const gb_server_config_t & cfg, gb_server * s) {
   GB_CUDA_TRY(cudaMalloc(&s->d_part, 2 * kMaxTiles * sizeof(double2)));
   s->slots.resize(cfg.max_slots);
   GB_CUDA_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+  GB_CUDA_TRY(cudaStreamCreateWithFlags(&s->copies, cudaStreamNonBlocking));
   GB_CUDA_TRY(cudaEventCreate(&s->step_start));
   GB_CUDA_TRY(cudaEventCreate(&s->step_done));
   GB_TRY(capture_graph(*s));
@@ -1176,7 +1179,7 @@ int admit(gb_server & s, Request & q, uint32_t k) {
   return GOOSEBERRY_SUCCESS;
 }
 
-// Enqueue a solve on the chip for slot k (the first, or with rounds > 0 the
+// Enqueue a launch of about slice_ns of a solve on the chip for slot k (the first, or with rounds > 0 the
 // correction A d = b - A x).  The caller holds its SMs.
 //
 // Nothing is queued behind the solve: the device's eight hardware queues are
@@ -1184,7 +1187,7 @@ int admit(gb_server & s, Request & q, uint32_t k) {
 // with an event behind each no more than eight solves ran at once.  The kernel
 // reports its end to the pinned block instead.  40 requests of 1k to 16k rows:
 // 23.4 -> 9.8 ms; 20 of 1k to 65k, mixed: 20.0 -> 16.4.
-int launch_on_chip(gb_server & s, uint32_t k) {
+int launch_on_chip(gb_server & s, uint32_t k, double slice_ns) {
   SlotHost & h = s.slots[k];
   const SrvSlot & S = h.dev;
   if (h.stream < 0) {
@@ -1218,7 +1221,7 @@ int launch_on_chip(gb_server & s, uint32_t k) {
   a.r_edge = h.r_edge;
   a.r_save = h.r_save;
   a.p_save = h.p_save[h.rounds ? 1 : 0];
-  resident_slice(&a, S.niter - h.iters, s.fault, h.resume ? &h.paused : nullptr);
+  resident_slice(&a, S.niter - h.iters, s.fault, slice_ns, h.resume ? &h.paused : nullptr);
   a.words = reinterpret_cast<unsigned long long *>(ctl);
   a.box = reinterpret_cast<ulonglong2 *>(ctl + kCtlBox);
   a.abort_flag = reinterpret_cast<int *>(ctl + kCtlFlag);
@@ -1532,27 +1535,23 @@ int cancel(gb_server & s, uint64_t id) {
   return GOOSEBERRY_ERROR_INVALIDINPUT;
 }
 
-int step(gb_server & s, size_t * active, size_t * queued) {
-  const auto t_in = std::chrono::steady_clock::now();
-  double waited = 0.0;
-  const bool drained = s.inflight;  // the wait below covers all earlier work on s.stream
-  if (s.inflight) {
-    GB_CUDA_TRY(cudaEventSynchronize(s.step_done));
-    waited = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_in)
-                 .count();
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, s.step_start, s.step_done) == cudaSuccess) s.stats.gpu_ms += ms;
-    s.stats.wait_ms += waited;
-    s.inflight = false;
-  }
-  if (!s.stage_done.empty()) {  // the admissions' copies ran before the replay waited on
-    if (!drained) GB_CUDA_TRY(cudaStreamSynchronize(s.stream));
-    for (const auto & r : s.stage_done) s.stage_alloc.release(r.first, r.second);
-    s.stage_done.clear();
-  }
-  // 0. collect the solves on the chip that have ended (a cancelled one stops
-  //    within 64 iterations)
-  bool moved = false, asked = false;
+// A result of slot k, whose solve is over; the slot and its memory are free then.
+void retire(gb_server & s, uint32_t k, gb_server_result_t res) {
+  SlotHost & h = s.slots[k];
+  res.id = h.id;
+  res.t_submit = h.t_submit;
+  res.t_admit = h.t_admit;
+  res.t_done = now_s(s);
+  s.results.push_back(res);
+  s.alloc.release(h.off, h.bytes);
+  h = SlotHost();
+}
+
+// Collect the solves on the chip that have ended (a cancelled one stops within
+// 64 iterations) and retire the finished or cancelled ones: x goes out on a
+// stream of its own, so that a replay under way does not hold it up.
+int collect_chip(gb_server & s, bool * moved) {
+  bool asked = false, any_done = false;
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
     if (h.used && h.chip == SlotHost::kRunning) {
@@ -1565,63 +1564,164 @@ int step(gb_server & s, size_t * active, size_t * queued) {
         }
         continue;
       }
+      // (the replay under way brings the slot table back: nothing joins it before)
+      if (pinned(s, k)->res.aborted && s.inflight) continue;
       GB_TRY(collect_on_chip(s, k));
-      moved = true;
+      *moved = true;
     }
     if (h.used && h.chip == SlotHost::kChecking) {
       const cudaError_t e = h.cancel ? cudaEventSynchronize(s.end[k]) : cudaEventQuery(s.end[k]);
       if (e == cudaErrorNotReady) continue;
       GB_CUDA_TRY(e);
       collect_residual(s, k);
-      moved = true;
+      *moved = true;
+    }
+    // a solve that finished before its cancel keeps x
+    if (h.used && h.chip == SlotHost::kFinished && h.status != GB_CG_CANCELLED) {
+      GB_CUDA_TRY(cudaMemcpyAsync(h.x_out, h.dev.x0, 8ull * h.n, cudaMemcpyDeviceToHost,
+          s.copies));
+      any_done = true;
     }
   }
-  // 1. retire finished (or cancelled) solves: copy x out, free memory and
-  //    the slot
+  if (any_done) GB_CUDA_TRY(cudaStreamSynchronize(s.copies));
+  for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
+    SlotHost & h = s.slots[k];
+    if (!h.used || !(h.chip == SlotHost::kFinished || (h.chip == SlotHost::kWaiting && h.cancel)))
+      continue;
+    gb_server_result_t res{};
+    res.iterations = h.iters + (h.resume ? h.paused.iter : 0);
+    res.refinements = h.rounds;
+    res.rnorm = h.resume ? std::sqrt(h.paused.rr) : h.rnorm;
+    res.bnorm = h.resume && h.rounds == 0 ? h.paused.bnorm : h.bnorm;
+    res.status = h.chip == SlotHost::kFinished ? h.status : GB_CG_CANCELLED;
+    if (h.copied) {
+      GB_CUDA_TRY(cudaEventSynchronize(h.copied));  // (cancelled before it was launched)
+      cudaEventDestroy(h.copied);
+    }
+    retire(s, k, res);
+    *moved = true;
+  }
+  return GOOSEBERRY_SUCCESS;
+}
+
+// Start solves on the chip while SMs are free, the longest waiting first; one
+// that does not fit lets later, smaller ones through for 20 ms, then SMs are kept
+// for it.  With solves in the batch a quarter of the SMs is the batch's, and a
+// solve that needs more than the rest takes turns with the replays: it is
+// launched, for 2 ms, while none is under way.  *first: the longest waiting one
+// that still waits (max_slots: none).
+int start_chip(gb_server & s, bool * launched, uint32_t * first) {
+  std::vector<uint32_t> wait;
+  bool batch = false;
+  for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
+    const SlotHost & h = s.slots[k];
+    if (h.used && h.chip == SlotHost::kWaiting && !h.cancel) wait.push_back(k);
+    batch |= h.used && h.chip == SlotHost::kBatch;
+  }
+  std::sort(wait.begin(), wait.end(), [&](uint32_t p, uint32_t q) {
+    return s.slots[p].t_admit != s.slots[q].t_admit ? s.slots[p].t_admit < s.slots[q].t_admit
+                                                    : p < q;
+  });
+  *first = s.cfg.max_slots;
+  const unsigned all = chip_capacity(s), rest = batch ? all - all / 4 : all;
+  for (uint32_t k : wait) {
+    SlotHost & h = s.slots[k];
+    const unsigned ctas = h.shape.args.ctas;
+    std::memset(&pinned(s, k)->res, 0, sizeof(ResResult));
+    resident_set_waits(&h.shape.args, s.fault, s.fault_limit_ms);
+    h.shape.fault = s.fault;
+    h.held = ctas > rest && s.inflight ? 0
+             : resident_try_acquire(s.device, ctas, ctas > rest ? all : rest,
+                   &pinned(s, k)->res.done);
+    if (!h.held) {
+      if (*first == s.cfg.max_slots) *first = k;
+      if (now_s(s) - h.t_admit > 0.02) break;
+      continue;
+    }
+    const int rc = launch_on_chip(s, k, ctas > rest ? 2e6 : kResSliceNs);
+    if (rc != GOOSEBERRY_SUCCESS) {
+      resident_release(s.device, h.held);
+      h.held = 0;
+      return rc;
+    }
+    *launched = true;
+  }
+  return GOOSEBERRY_SUCCESS;
+}
+
+int step(gb_server & s, size_t * active, size_t * queued) {
+  const auto t_in = std::chrono::steady_clock::now();
+  const auto ms_since = [](std::chrono::steady_clock::time_point t) {
+    return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count();
+  };
+  double waited = 0.0;
+  bool moved = false, launched = false;
+  uint32_t first = s.cfg.max_slots;
+  const bool drained = s.inflight;  // the wait below covers all earlier work on s.stream
+  if (s.inflight) {
+    // The replay under way may wait for SMs that solves on the chip hold, its own
+    // server's or others', so those are served meanwhile, and after a millisecond
+    // the caller has its turn.
+    cudaError_t e = cudaEventQuery(s.step_done);
+    while (e == cudaErrorNotReady) {
+      bool chip = false;
+      for (const auto & h : s.slots) chip |= h.used && h.chip != SlotHost::kBatch;
+      if (!chip) {
+        e = cudaEventSynchronize(s.step_done);
+        break;
+      }
+      GB_TRY(collect_chip(s, &moved));
+      GB_TRY(start_chip(s, &launched, &first));
+      e = cudaEventQuery(s.step_done);
+      if (ms_since(t_in) > 1.0) break;
+    }
+    waited = ms_since(t_in);
+    s.stats.wait_ms += waited;
+    if (e == cudaErrorNotReady) {
+      if (launched) s.stats.steps += 1;
+      if (active) *active = std::count_if(s.slots.begin(), s.slots.end(),
+                                          [](const SlotHost & h) { return h.used; });
+      if (queued) *queued = s.queue.size();
+      return GOOSEBERRY_SUCCESS;
+    }
+    GB_CUDA_TRY(e);
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, s.step_start, s.step_done) == cudaSuccess) s.stats.gpu_ms += ms;
+    s.inflight = false;
+  }
+  if (!s.stage_done.empty()) {  // the admissions' copies ran before the replay waited on
+    if (!drained) GB_CUDA_TRY(cudaStreamSynchronize(s.stream));
+    for (const auto & r : s.stage_done) s.stage_alloc.release(r.first, r.second);
+    s.stage_done.clear();
+  }
+  // 0. the solves on the chip
+  GB_TRY(collect_chip(s, &moved));
+  // 1. retire the batch's finished (or cancelled) solves: copy x out, free memory
+  //    and the slot
   bool any_done = false;
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
     const SrvSlot & S = s.h_slots[k];
-    const bool on_chip = h.chip == SlotHost::kFinished && h.status != GB_CG_CANCELLED;
     // a solve that finished before its cancel keeps x
-    if (!h.used || !(h.chip == SlotHost::kBatch ? S.done != 0 : on_chip)) continue;
-    const double * x = on_chip ? h.dev.x0 : (s.mixed && S.xpar) ? S.x1 : S.x0;
-    GB_CUDA_TRY(cudaMemcpyAsync(h.x_out, x, 8ull * h.n, cudaMemcpyDeviceToHost, s.stream));
+    if (!h.used || h.chip != SlotHost::kBatch || !S.done) continue;
+    GB_CUDA_TRY(cudaMemcpyAsync(h.x_out, (s.mixed && S.xpar) ? S.x1 : S.x0, 8ull * h.n,
+        cudaMemcpyDeviceToHost, s.stream));
     any_done = true;
   }
   if (any_done) GB_CUDA_TRY(cudaStreamSynchronize(s.stream));
   for (uint32_t k = 0; k < s.cfg.max_slots; ++k) {
     SlotHost & h = s.slots[k];
     SrvSlot & S = s.h_slots[k];
-    const bool batch = h.chip == SlotHost::kBatch;
-    if (!h.used || !((batch ? S.done != 0 : h.chip == SlotHost::kFinished) || h.cancel)) continue;
-    gb_server_result_t res;
-    res.id = h.id;
-    if (batch) {
-      res.iterations = S.iter;
-      res.refinements = S.refinements;
-      res.rnorm = std::sqrt(S.rr_true);
-      res.bnorm = S.bnorm;
-      res.status = S.done ? S.status : GB_CG_CANCELLED;
-    } else {
-      res.iterations = h.iters + (h.resume ? h.paused.iter : 0);
-      res.refinements = h.rounds;
-      res.rnorm = h.resume ? std::sqrt(h.paused.rr) : h.rnorm;
-      res.bnorm = h.resume && h.rounds == 0 ? h.paused.bnorm : h.bnorm;
-      res.status = h.chip == SlotHost::kFinished ? h.status : GB_CG_CANCELLED;
-      if (h.copied) {
-        GB_CUDA_TRY(cudaEventSynchronize(h.copied));  // (cancelled before it was launched)
-        cudaEventDestroy(h.copied);
-      }
-    }
-    res.t_submit = h.t_submit;
-    res.t_admit = h.t_admit;
-    res.t_done = now_s(s);
-    s.results.push_back(res);
-    s.alloc.release(h.off, h.bytes);
-    if (batch) s.dirty = true;
-    h = SlotHost();
+    if (!h.used || h.chip != SlotHost::kBatch || !(S.done || h.cancel)) continue;
+    gb_server_result_t res{};
+    res.iterations = S.iter;
+    res.refinements = S.refinements;
+    res.rnorm = std::sqrt(S.rr_true);
+    res.bnorm = S.bnorm;
+    res.status = S.done ? S.status : GB_CG_CANCELLED;
+    retire(s, k, res);
     std::memset(&S, 0, sizeof(S));
+    s.dirty = true;
     moved = true;
   }
   // 2. admit queued requests (FIFO; a request that does not fit yet lets a
@@ -1644,48 +1744,19 @@ int step(gb_server & s, size_t * active, size_t * queued) {
     it = s.queue.erase(it);
     moved = true;
   }
-  // 2b. start solves on the chip while SMs are free, the longest waiting first;
-  //     one that does not fit lets later, smaller ones through for 20 ms, then
-  //     SMs are kept for it
-  bool launched = false;
-  std::vector<uint32_t> wait;
-  for (uint32_t k = 0; k < s.cfg.max_slots; ++k)
-    if (s.slots[k].used && s.slots[k].chip == SlotHost::kWaiting && !s.slots[k].cancel)
-      wait.push_back(k);
-  std::sort(wait.begin(), wait.end(), [&](uint32_t p, uint32_t q) {
-    return s.slots[p].t_admit != s.slots[q].t_admit ? s.slots[p].t_admit < s.slots[q].t_admit
-                                                    : p < q;
-  });
-  for (uint32_t k : wait) {
-    SlotHost & h = s.slots[k];
-    std::memset(&pinned(s, k)->res, 0, sizeof(ResResult));
-    resident_set_waits(&h.shape.args, s.fault, s.fault_limit_ms);
-    h.shape.fault = s.fault;
-    h.held = resident_try_acquire(s.device, h.shape.args.ctas, chip_capacity(s),
-        &pinned(s, k)->res.done);
-    if (!h.held) {
-      if (now_s(s) - h.t_admit > 0.02) break;
-      continue;
-    }
-    const int rc = launch_on_chip(s, k);
-    if (rc != GOOSEBERRY_SUCCESS) {
-      resident_release(s.device, h.held);
-      h.held = 0;
-      return rc;
-    }
-    launched = true;
-  }
+  // 2b. start solves on the chip
+  GB_TRY(start_chip(s, &launched, &first));
   // nothing of this server runs on the chip, and others have not left the SMs to
   // the longest waiting request for as long as any wait may take: the batch
   bool on_chip = false;
   for (const auto & h : s.slots)
     on_chip |= h.used && (h.chip == SlotHost::kRunning || h.chip == SlotHost::kChecking);
-  if (wait.empty() || on_chip) {
+  if (first == s.cfg.max_slots || on_chip) {
     s.starved_since = -1.0;
   } else if (s.starved_since < 0.0) {
     s.starved_since = now_s(s);
-  } else if (now_s(s) - s.starved_since > 1e-9 * s.slots[wait[0]].shape.args.wait_ns) {
-    GB_TRY(to_batch(s, wait[0]));
+  } else if (now_s(s) - s.starved_since > 1e-9 * s.slots[first].shape.args.wait_ns) {
+    GB_TRY(to_batch(s, first));
     s.starved_since = -1.0;
     moved = true;
   }
@@ -1721,7 +1792,7 @@ int step(gb_server & s, size_t * active, size_t * queued) {
   if (launched && !nbatch) s.stats.steps += 1;
   // with nothing to do but wait for solves on the chip, wait for one (at most
   // a millisecond, so that a caller's submissions and cancels get their turn)
-  if (!running && !wait.empty() && !nbatch && !moved) {
+  if (!running && first < s.cfg.max_slots && !nbatch && !moved) {
     std::this_thread::sleep_for(std::chrono::microseconds(200));  // others hold the SMs
     s.stats.wait_ms += 0.2;
     waited += 0.2;

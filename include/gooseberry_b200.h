@@ -401,9 +401,9 @@ GOOSEBERRY_API int gb_cg_row_bytes(const gb_cg_t * s, size_t * bytes);
 /*
  * Many independent CG solves of uneven sizes resident on one GPU at once.
  * Requests whose systems fit the SMs' shared memory (stencils: at most 7
- * entries a row, at most 256 lists of column offsets) are each solved by one
- * launch on as many SMs as they need, started by gb_server_step as SMs come
- * free (in FP64 also under GB_CG_MIXED, which judges them on b - A x); the
+ * entries a row, at most 256 lists of column offsets) are each solved by launches
+ * of about 10 ms on as many SMs as they need, started by gb_server_step as SMs
+ * come free (in FP64 also under GB_CG_MIXED, which judges them on b - A x); the
  * batch serves the others.
  * Every gb_server_step runs `iters_per_step` CG iterations of EVERY batched
  * solve with one replay of a captured CUDA graph (the kernels walk a global
@@ -456,8 +456,10 @@ GOOSEBERRY_API int gb_server_submit(gb_server_t * s, uint64_t id, dim_t n,
     double * x_out, double tol_rel, size_t niter);
 
 /* One scheduling step (see above).  Returns at once after queueing the
- * step's GPU work; with nothing to queue while solves run on the chip, it
- * waits for one of them to end, at most a millisecond.  *active / *queued (optional) receive the resident and
+ * step's GPU work.  While solves run on the chip it waits at most a
+ * millisecond: for one of them to end when there is nothing to queue, or for
+ * the batch's last replay, serving them meanwhile (a replay that is not done
+ * by then goes on; a later step takes its results).  *active / *queued (optional) receive the resident and
  * waiting request counts. */
 GOOSEBERRY_API int gb_server_step(gb_server_t * s, size_t * active, size_t * queued);
 
