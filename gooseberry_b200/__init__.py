@@ -57,6 +57,7 @@ CG_F64, CG_MIXED = 0, 1
 CG_PERSISTENT = 0x100
 CG_PLAIN_ENTRIES = 0x200
 CHIP_FAULT_NONE, CHIP_FAULT_MISSING, CHIP_FAULT_LATE, CHIP_FAULT_SHORT = 0, 1, 2, 3
+CHIP_FAULT_REFUSED = 4
 CG_STATUS = {0: "converged", 1: "maxiter", 2: "breakdown", 3: "nonfinite", 4: "cancelled",
              5: "timeout"}
 
@@ -705,7 +706,8 @@ class CgSolver:
         of the following solves is missing (``CHIP_FAULT_MISSING``) or late
         (``CHIP_FAULT_LATE``), so they are given up after ``limit_ms`` (0: the 2 s
         default) and run by the graph-replayed kernels; or every launch ends at
-        its first check of the time and the next goes on (``CHIP_FAULT_SHORT``)."""
+        its first check of the time and the next goes on (``CHIP_FAULT_SHORT``), or
+        is taken as turned down by the driver (``CHIP_FAULT_REFUSED``)."""
         _check(lib().gb_cg_set_chip_fault(self._h, int(fault), int(limit_ms)),
                "gb_cg_set_chip_fault")
 

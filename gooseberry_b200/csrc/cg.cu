@@ -1905,7 +1905,7 @@ int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned limit_ms) {
 
 int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms) {
   GB_CHECK_INPUT(s != nullptr, "solver is NULL");
-  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_SHORT, "unknown fault %d",
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_REFUSED, "unknown fault %d",
       fault);
   GB_CHECK_INPUT(s->resident && gb::resident_set_fault(s->resident, fault, limit_ms),
       "the fault applies to solves on the chip by more than one CTA");

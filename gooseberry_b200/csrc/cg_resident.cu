@@ -1003,10 +1003,26 @@ int resident_preload() {
   return GOOSEBERRY_SUCCESS;
 }
 
-int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream) {
-  void * kargs[] = {&args};
-  GB_CUDA_TRY(cudaLaunchCooperativeKernel(sh.fn, dim3(resident_grid(args, sh.fault)), dim3(sh.threads), kargs, sh.smem,
-      stream));
+// A cooperative launch that the driver turns down (the SMs that this process may
+// use do not hold the grid) leaves the device as it was.
+static cudaError_t resident_start(const void * fn, int threads, size_t smem, ResArgs * args,
+    int fault, cudaStream_t stream, bool * refused) {
+  void * kargs[] = {args};
+  cudaError_t e = fault == GB_CHIP_FAULT_REFUSED
+      ? cudaErrorCooperativeLaunchTooLarge
+      : cudaLaunchCooperativeKernel(fn, dim3(resident_grid(*args, fault)), dim3(threads), kargs,
+            smem, stream);
+  *refused = e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+             e == cudaErrorNotSupported || e == cudaErrorNotPermitted;
+  if (*refused) {
+    cudaGetLastError();
+    e = cudaSuccess;
+  }
+  return e;
+}
+
+int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream, bool * refused) {
+  GB_CUDA_TRY(resident_start(sh.fn, sh.threads, sh.smem, &args, sh.fault, stream, refused));
   return GOOSEBERRY_SUCCESS;
 }
 
@@ -1221,9 +1237,9 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
       return GOOSEBERRY_SUCCESS;
     }
     std::memset(s->out_h, 0, sizeof(ResResult));
-    void * kargs[] = {&g};
-    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(s->fn),
-        dim3(resident_grid(g, s->fault)), dim3(s->threads), kargs, s->smem, stream);
+    bool refused = false;
+    cudaError_t e = resident_start(reinterpret_cast<const void *>(s->fn), s->threads, s->smem, &g,
+        s->fault, stream, &refused);
     const cudaError_t e2 = cudaStreamSynchronize(stream);
     resident_release(s->a->device, held);
     if (e == cudaSuccess) e = e2;
@@ -1232,6 +1248,7 @@ int resident_solve(ResidentCg * s, const double * b, double tol, int tol_relativ
       set_error("CG solve failed: %s", cudaGetErrorString(e));
       return GOOSEBERRY_ERROR_UNKNOWN;
     }
+    if (refused) s->out_h->aborted = 1;  // nothing ran
     res->result = *s->out_h;
     ++res->launches;
     // an abandoned solve leaves the CTAs at different counts

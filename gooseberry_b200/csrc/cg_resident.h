@@ -133,7 +133,7 @@ int resident_shape(uint32_t n, uint32_t half, int max_row, uint32_t npat, int sm
 int resident_preload();
 // Enqueue a solve.  The caller holds the grid's SMs (resident_try_acquire) until
 // it has ended, and has cleared words, box, abort flag and r_edge.
-int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream);
+int resident_launch(const ResShape & sh, ResArgs args, cudaStream_t stream, bool * refused);
 constexpr int kResMaxCtas = 160;  // tagged partials polled, 5 a lane
 
 // r = b - A x and r.r into *rr (may be host-mapped), with `grid` partials and a

@@ -1187,7 +1187,7 @@ int admit(gb_server & s, Request & q, uint32_t k) {
 // with an event behind each no more than eight solves ran at once.  The kernel
 // reports its end to the pinned block instead.  40 requests of 1k to 16k rows:
 // 23.4 -> 9.8 ms; 20 of 1k to 65k, mixed: 20.0 -> 16.4.
-int launch_on_chip(gb_server & s, uint32_t k, double slice_ns) {
+int launch_on_chip(gb_server & s, uint32_t k, double slice_ns, bool * refused) {
   SlotHost & h = s.slots[k];
   const SrvSlot & S = h.dev;
   if (h.stream < 0) {
@@ -1229,7 +1229,8 @@ int launch_on_chip(gb_server & s, uint32_t k, double slice_ns) {
   a.out = &pinned_dev(s, k)->res;
   a.epoch0 = 2;
   a.arrived = reinterpret_cast<unsigned *>(ctl + kCtlFlag + 32);
-  GB_TRY(resident_launch(h.shape, a, st));
+  GB_TRY(resident_launch(h.shape, a, st, refused));
+  if (*refused) return GOOSEBERRY_SUCCESS;
   h.chip = SlotHost::kRunning;
   return GOOSEBERRY_SUCCESS;
 }
@@ -1638,11 +1639,14 @@ int start_chip(gb_server & s, bool * launched, uint32_t * first) {
       if (now_s(s) - h.t_admit > 0.02) break;
       continue;
     }
-    const int rc = launch_on_chip(s, k, ctas > rest ? 2e6 : kResSliceNs);
-    if (rc != GOOSEBERRY_SUCCESS) {
+    bool refused = false;
+    const int rc = launch_on_chip(s, k, ctas > rest ? 2e6 : kResSliceNs, &refused);
+    if (rc != GOOSEBERRY_SUCCESS || refused) {
       resident_release(s.device, h.held);
       h.held = 0;
-      return rc;
+      GB_TRY(rc);
+      if (!s.inflight) GB_TRY(to_batch(s, k));
+      continue;
     }
     *launched = true;
   }
@@ -1900,7 +1904,7 @@ int gb_server_cancel(gb_server_t * s, uint64_t id) {
 
 int gb_server_set_chip_fault(gb_server_t * s, int fault, unsigned limit_ms) {
   GB_CHECK_INPUT(s != nullptr, "server is NULL");
-  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_SHORT, "unknown fault %d",
+  GB_CHECK_INPUT(fault >= GB_CHIP_FAULT_NONE && fault <= GB_CHIP_FAULT_REFUSED, "unknown fault %d",
       fault);
   s->fault = fault;
   s->fault_limit_ms = limit_ms;

@@ -355,14 +355,16 @@ GOOSEBERRY_API int gb_cg_set_barrier_fault(gb_cg_t * s, int drop_cta, unsigned l
  * up when the limit is over, raise the abort flag and leave (as a late one then
  * does), and the call runs the solve by the graph-replayed kernels and returns
  * their result.  With SHORT every launch of a solve ends at its first check of
- * the time, some 64 iterations, and the next goes on.  `limit_ms` sets the limit (0: 2000).  Nothing waits without
+ * the time, some 64 iterations, and the next goes on.  With REFUSED launches are taken as
+ * turned down by the driver, and the graph-replayed kernels run the solve.  `limit_ms` sets the limit (0: 2000).  Nothing waits without
  * one, so the device stays usable.  Refused for a solver that does not solve on
  * the chip, or that does on one CTA.  No reference counterpart. */
 typedef enum gb_chip_fault {
   GB_CHIP_FAULT_NONE = 0,
   GB_CHIP_FAULT_MISSING = 1,
   GB_CHIP_FAULT_LATE = 2,
-  GB_CHIP_FAULT_SHORT = 3
+  GB_CHIP_FAULT_SHORT = 3,
+  GB_CHIP_FAULT_REFUSED = 4
 } gb_chip_fault_t;
 GOOSEBERRY_API int gb_cg_set_chip_fault(gb_cg_t * s, int fault, unsigned limit_ms);
 
