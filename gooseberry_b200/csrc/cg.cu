@@ -1669,7 +1669,7 @@ int solve_cg(gb_cg * s, const double * b, double * x, double tol, int tol_relati
     cudaStream_t stream) {
   if (s->mixed) {
     if (s->resident) {
-      GB_CHECK_INPUT(b && x, "NULL vector");
+      GB_TRY(mixed_check(s->mixed, b, x));
       bool done = false;
       GB_TRY(solve_resident(s, b, x, tol, tol_relative, niter, history, history_len, res, stream,
           &done));

@@ -1163,13 +1163,18 @@ int mixed_start(MixedCg * m, const double * b, double tol, int tol_relative, siz
 
 }  // namespace
 
-int mixed_solve(MixedCg * m, const double * b, double * x, double tol, int tol_relative,
-    size_t niter, double * history, size_t history_len, gb_cg_result_t * res,
-    cudaStream_t stream, const int * cancel) {
+int mixed_check(const MixedCg * m, const double * b, const double * x) {
   GB_CHECK_INPUT(m->n == 0 || (b && x), "NULL vector");
   GB_CHECK_INPUT(m->a->sched32 == m->sched32 && m->a->sched64 == m->sched64 &&
                  m->a->plan.tile_items == m->tile_items,
       "matrix schedule changed after the solver was created");
+  return GOOSEBERRY_SUCCESS;
+}
+
+int mixed_solve(MixedCg * m, const double * b, double * x, double tol, int tol_relative,
+    size_t niter, double * history, size_t history_len, gb_cg_result_t * res,
+    cudaStream_t stream, const int * cancel) {
+  GB_TRY(mixed_check(m, b, x));
   if (m->n == 0) {
     if (res) *res = gb_cg_result_t{0, 0, 0.0, 0.0, GB_CG_CONVERGED, 0};
     return GOOSEBERRY_SUCCESS;

@@ -285,6 +285,8 @@ int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out);
 // Lay a symmetric pattern matrix that exceeds L2 out by its diagonals
 // (SymDiags): for a solver whose solves do not run on the chip.
 int mixed_past_chip(MixedCg * m);
+// What a solve needs: its vectors, and the matrix's schedules as at creation.
+int mixed_check(const MixedCg * m, const double * b, const double * x);
 size_t mixed_entry_bytes(const MixedCg * m);
 size_t mixed_row_bytes(const MixedCg * m);
 void mixed_destroy(MixedCg * m);
