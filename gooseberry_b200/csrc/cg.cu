@@ -1280,6 +1280,11 @@ int setup_resident(const gb_csr * a, bool plain, gb_cg * s) {
   return rc;
 }
 
+void drop_resident(gb_cg * s) {
+  resident_destroy(s->resident);
+  s->resident = nullptr;
+}
+
 // One cooperative launch per solve when every row fits a tile (no long rows)
 // and all CTAs of the grid can be resident at once.  Tiles are dealt to CTAs
 // in contiguous runs of nearly equal rows + nonzeros.
@@ -1354,6 +1359,50 @@ int launch_persistent(gb_cg * s, const double * b, int tol_relative, cudaStream_
   return GOOSEBERRY_SUCCESS;
 }
 
+// A GB_CG_MIXED system whose FP64 vectors fit the chip is solved there in FP64:
+// its iterations wait for exchanges and shared memory, not for the bytes that
+// floats would save, and convergence is still judged on b - A x.  Where it does
+// not fit (too wide a band, or no device memory for it) nothing of it is kept,
+// and the solver has its FP32 iterations alone.
+bool try_mixed_on_chip(const gb_csr * a, bool plain_entries, gb_cg * s) {
+  if (a->sched64 != GB_SCHED_ROW || a->nnz == 0 || !resident_size_ok(*a)) return false;
+  const auto setup = [&]() -> int {
+    GB_TRY(dev_alloc(&s->x, std::max<size_t>(s->n, 2) * sizeof(double)));
+    if (!plain_entries) {
+      GB_TRY(build_row_codec(*a, &s->codec, nullptr));
+      GB_TRY(build_ell(a, s));
+    }
+    GB_TRY(setup_resident(a, plain_entries, s));
+    if (!s->resident) return GOOSEBERRY_SUCCESS;
+    GB_TRY(dev_alloc(&s->r, s->n * sizeof(double)));
+    GB_TRY(dev_alloc(&s->xsum, s->n * sizeof(double)));
+    GB_TRY(dev_alloc(&s->partial_a, static_cast<size_t>(a->sm_count) * 4 * sizeof(double)));
+    GB_TRY(dev_alloc(&s->ticket, sizeof(unsigned)));
+    GB_CUDA_TRY(cudaMemset(s->ticket, 0, sizeof(unsigned)));
+    return pinned_slot_alloc(sizeof(double), reinterpret_cast<void **>(&s->rr_true_h),
+        reinterpret_cast<void **>(&s->rr_true_d));
+  };
+  if (setup() == GOOSEBERRY_SUCCESS && s->resident) return true;
+  cudaGetLastError();
+  cudaDeviceSynchronize();  // its memory goes back to the pool
+  drop_resident(s);
+  free_row_codec(s->codec);
+  free_row_patterns(s->pat);
+  const auto drop = [](auto *& p) {
+    dev_free(p);
+    p = nullptr;
+  };
+  drop(s->ell8);
+  dev_free(s->ellv);
+  s->ellv = nullptr;
+  drop(s->x);
+  drop(s->r);
+  drop(s->xsum);
+  drop(s->partial_a);
+  drop(s->ticket);
+  return false;
+}
+
 int create_cg(const gb_csr * a, int mode, gb_cg * s) {
   GB_CHECK_INPUT(a->nrows == a->ncols, "CG needs a square matrix, got %ux%u", a->nrows,
       a->ncols);
@@ -1368,35 +1417,11 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
     s->mode = mode;
     s->n = a->nrows;
     GB_TRY(mixed_create(a, plain_entries, &s->mixed));
-    // A system whose FP64 vectors fit the chip is solved there in FP64: its
-    // iterations wait for exchanges and shared memory, not for the bytes that
-    // floats would save, and convergence is still judged on b - A x.
-    if (a->sched64 != GB_SCHED_ROW || a->nnz == 0 || !resident_size_ok(*a))
-      return mixed_past_chip(s->mixed);
-    GB_TRY(dev_alloc(&s->x, std::max<size_t>(s->n, 2) * sizeof(double)));
-    if (!plain_entries) {
-      GB_TRY(build_row_codec(*a, &s->codec, nullptr));
-      GB_TRY(build_ell(a, s));
+    if (!try_mixed_on_chip(a, plain_entries, s)) {
+      GB_TRY(mixed_past_chip(s->mixed));
+      GB_TRY(mixed_ensure_graphs(s->mixed));
     }
-    GB_TRY(setup_resident(a, plain_entries, s));
-    if (!s->resident) {  // too wide a band: nothing of this is used
-      free_row_codec(s->codec);
-      free_row_patterns(s->pat);
-      dev_free(s->ell8);
-      dev_free(s->ellv);
-      dev_free(s->x);
-      s->ell8 = nullptr;
-      s->ellv = nullptr;
-      s->x = nullptr;
-      return GOOSEBERRY_SUCCESS;
-    }
-    GB_TRY(dev_alloc(&s->r, s->n * sizeof(double)));
-    GB_TRY(dev_alloc(&s->xsum, s->n * sizeof(double)));
-    GB_TRY(dev_alloc(&s->partial_a, static_cast<size_t>(a->sm_count) * 4 * sizeof(double)));
-    GB_TRY(dev_alloc(&s->ticket, sizeof(unsigned)));
-    GB_CUDA_TRY(cudaMemset(s->ticket, 0, sizeof(unsigned)));
-    return pinned_slot_alloc(sizeof(double), reinterpret_cast<void **>(&s->rr_true_h),
-        reinterpret_cast<void **>(&s->rr_true_d));
+    return GOOSEBERRY_SUCCESS;
   }
   GB_CHECK_INPUT(a->val64 != nullptr, "CG (FP64) needs double values on the matrix");
   s->a = a;
@@ -1457,7 +1482,10 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
   GB_TRY(pinned_slot_alloc(2 * sizeof(CgStatus), reinterpret_cast<void **>(&s->host_status),
       nullptr));
   if (want_persistent) GB_TRY(setup_persistent(a, s));
-  else if (s->sched == GB_SCHED_ROW) GB_TRY(setup_resident(a, plain_entries, s));
+  else if (s->sched == GB_SCHED_ROW && setup_resident(a, plain_entries, s) != GOOSEBERRY_SUCCESS) {
+    cudaGetLastError();  // no memory for the solve on the chip
+    drop_resident(s);
+  }
   if (!s->persistent && !s->resident) GB_TRY(ensure_graphs(s));
   return GOOSEBERRY_SUCCESS;
 }

@@ -1111,10 +1111,15 @@ int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out) {
   GB_CUDA_TRY(cudaMemset(m->st, 0, sizeof(MixState)));
   GB_TRY(pinned_slot_alloc(2 * sizeof(MixStatus), reinterpret_cast<void **>(&m->host_status),
       nullptr));
-  GB_CUDA_TRY(cudaStreamCreateWithFlags(&m->cap_stream, cudaStreamNonBlocking));
-  GB_TRY(capture(m, 0));
-  GB_TRY(capture(m, 1));
   return GOOSEBERRY_SUCCESS;
+}
+
+int mixed_ensure_graphs(MixedCg * m) {
+  if (m->graph[1]) return GOOSEBERRY_SUCCESS;
+  if (!m->cap_stream)
+    GB_CUDA_TRY(cudaStreamCreateWithFlags(&m->cap_stream, cudaStreamNonBlocking));
+  if (!m->graph[0]) GB_TRY(capture(m, 0));
+  return capture(m, 1);
 }
 
 int mixed_past_chip(MixedCg * m) {
@@ -1133,13 +1138,7 @@ int mixed_past_chip(MixedCg * m) {
   }
   dev_free(m->v8);
   m->v8 = nullptr;
-  for (auto & g : m->graph) {  // captured over the rows of 8
-    if (g) cudaGraphExecDestroy(g);
-    g = nullptr;
-  }
-  GB_TRY(l2_fits(mixed_row_bytes(m) * (m->n + 1) + 24ull * m->n, &m->l2_hint));
-  GB_TRY(capture(m, 0));
-  return capture(m, 1);
+  return l2_fits(mixed_row_bytes(m) * (m->n + 1) + 24ull * m->n, &m->l2_hint);
 }
 
 namespace {
@@ -1179,6 +1178,7 @@ int mixed_solve(MixedCg * m, const double * b, double * x, double tol, int tol_r
     if (res) *res = gb_cg_result_t{0, 0, 0.0, 0.0, GB_CG_CONVERGED, 0};
     return GOOSEBERRY_SUCCESS;
   }
+  GB_TRY(mixed_ensure_graphs(m));
   double * dhist = nullptr;
   const size_t hl = history ? std::min(history_len, niter ? niter : history_len) : 0;
   if (hl) GB_TRY(scratch_alloc(reinterpret_cast<void **>(&dhist), hl * sizeof(double), stream));

@@ -283,8 +283,12 @@ int row_stage_for(const gb_csr & a);
 struct MixedCg;
 int mixed_create(const gb_csr * a, bool plain_entries, MixedCg ** out);
 // Lay a symmetric pattern matrix that exceeds L2 out by its diagonals
-// (SymDiags): for a solver whose solves do not run on the chip.
+// (SymDiags): for a solver whose solves do not run on the chip.  Before its
+// graphs are captured.
 int mixed_past_chip(MixedCg * m);
+// The two chunk graphs, captured at creation, or on first use by a solver whose
+// solves run on the chip.
+int mixed_ensure_graphs(MixedCg * m);
 // What a solve needs: its vectors, and the matrix's schedules as at creation.
 int mixed_check(const MixedCg * m, const double * b, const double * x);
 size_t mixed_entry_bytes(const MixedCg * m);
