@@ -56,6 +56,7 @@ SCHED_NAMES = {0: "auto", 1: "thread", 2: "group4", 3: "group8", 4: "warp", 5: "
 CG_F64, CG_MIXED = 0, 1
 CG_PERSISTENT = 0x100
 CG_PLAIN_ENTRIES = 0x200
+ROWS_PLAIN, ROWS_PATTERNS, ROWS_CLASSES = 0, 1, 2
 CHIP_FAULT_NONE, CHIP_FAULT_MISSING, CHIP_FAULT_LATE, CHIP_FAULT_SHORT = 0, 1, 2, 3
 CHIP_FAULT_REFUSED = 4
 CG_STATUS = {0: "converged", 1: "maxiter", 2: "breakdown", 3: "nonfinite", 4: "cancelled",
@@ -123,6 +124,8 @@ SIGNATURES = {
     "gb_csr_get_info": (_i, [_vp, _vp]),
     "gb_csr_set_schedule": (_i, [_vp, C.c_uint, _i, _u32]),
     "gb_csr_autotune": (_i, [_vp, C.c_uint, _vp]),
+    "gb_csr_row_form": (_i, [_vp, C.c_uint, _vp]),
+    "gb_csr_compress_rows": (_i, [_vp, C.c_uint]),
     "gb_plan_tiles_host": (_i, [_u32, _vp, _u32, _u32, _vp, _sz, _vp, _vp, _vp]),
     "gb_spmv_f64": (_i, [_vp, _vp, _vp, _vp]),
     "gb_spmv_f32": (_i, [_vp, _vp, _vp, _vp]),
@@ -596,6 +599,20 @@ class CsrMatrix:
     def set_schedule(self, schedule: int, tile_items: int = 0, f32: bool = False):
         _check(lib().gb_csr_set_schedule(self._h, VALUES_F32 if f32 else VALUES_F64,
                                          schedule, tile_items), "gb_csr_set_schedule")
+
+    def row_form(self, f32: bool = False) -> int:
+        """What the row schedule reads (``gb_csr_row_form``): ``ROWS_PLAIN``,
+        ``ROWS_PATTERNS`` or ``ROWS_CLASSES``."""
+        v = C.c_int(0)
+        _check(lib().gb_csr_row_form(self._h, VALUES_F32 if f32 else VALUES_F64,
+                                     C.addressof(v)), "gb_csr_row_form")
+        return v.value
+
+    def compress_rows(self, f32: bool = False):
+        """The row schedule over the matrix's compressed copy
+        (``gb_csr_compress_rows``)."""
+        _check(lib().gb_csr_compress_rows(self._h, VALUES_F32 if f32 else VALUES_F64),
+               "gb_csr_compress_rows")
 
     def autotune(self, f32: bool = False, stream=None):
         _check(lib().gb_csr_autotune(self._h, VALUES_F32 if f32 else VALUES_F64,

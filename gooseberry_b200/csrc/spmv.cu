@@ -647,12 +647,17 @@ int preload_round_f32() {
 
 namespace {
 
+int pattern_form(const SpmvPattern * p) {
+  return !p ? GB_ROWS_PLAIN : p->cls.code8 ? GB_ROWS_CLASSES : GB_ROWS_PATTERNS;
+}
+
 struct TuneKey {
   uint32_t p50, p90, p99, maxlog2, nrows_log2, nnz_log2;
   unsigned width;
+  int form;  // of its compressed copy (gb_row_form_t): each is timed on its own
   bool operator<(const TuneKey & o) const {
-    return std::tie(p50, p90, p99, maxlog2, nrows_log2, nnz_log2, width) <
-           std::tie(o.p50, o.p90, o.p99, o.maxlog2, o.nrows_log2, o.nnz_log2, o.width);
+    return std::tie(p50, p90, p99, maxlog2, nrows_log2, nnz_log2, width, form) <
+           std::tie(o.p50, o.p90, o.p99, o.maxlog2, o.nrows_log2, o.nnz_log2, o.width, o.form);
   }
 };
 struct TuneChoice {
@@ -665,7 +670,7 @@ std::map<TuneKey, TuneChoice> g_tune_cache;
 
 uint32_t ilog2(uint64_t v) { return v ? 63u - static_cast<uint32_t>(__builtin_clzll(v)) : 0u; }
 
-TuneKey make_key(const gb_csr & a, unsigned width) {
+TuneKey make_key(const gb_csr & a, unsigned width, const SpmvPattern * p) {
   TuneKey k;
   k.p50 = a.plan.p50;
   k.p90 = a.plan.p90;
@@ -674,6 +679,7 @@ TuneKey make_key(const gb_csr & a, unsigned width) {
   k.nrows_log2 = ilog2(a.nrows);
   k.nnz_log2 = ilog2(a.nnz);
   k.width = width;
+  k.form = pattern_form(p);
   return k;
 }
 
@@ -738,27 +744,49 @@ void drop_pattern(gb_csr & a, unsigned width) {
 int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   SpmvPattern *& pattern = width == GB_CSR_VALUES_F32 ? a.pat32 : a.pat64;
   drop_pattern(a, width);
-  const TuneKey key = make_key(a, width);
+  const bool short_rows = a.plan.p99 <= 64 && a.plan.max_row <= 4096;
+  SpmvPattern * trial = nullptr;
+  if (short_rows) GB_TRY(build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &trial, stream));
+  const auto drop_trial = [&] {
+    if (!trial) return;
+    cudaStreamSynchronize(stream);
+    free_spmv_pattern(trial);
+    trial = nullptr;
+  };
+  const TuneKey key = make_key(a, width, trial);
+  TuneChoice known{};
+  bool hit = false;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end()) {
-      GB_TRY(rebuild_plan(a, it->second.tile_items, stream));
-      if (it->second.sched == GB_SCHED_SEG) GB_TRY(ensure_seg_plan(a, stream));
-      (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = it->second.sched;
-      // (a matrix of this shape without patterns keeps the plain row schedule)
-      return it->second.pattern
-                 ? build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &pattern, stream)
-                 : GOOSEBERRY_SUCCESS;
-    }
+    if ((hit = it != g_tune_cache.end())) known = it->second;
+  }
+  if (hit) {
+    int rc = rebuild_plan(a, known.tile_items, stream);
+    if (rc == GOOSEBERRY_SUCCESS && known.sched == GB_SCHED_SEG) rc = ensure_seg_plan(a, stream);
+    if (rc != GOOSEBERRY_SUCCESS || !known.pattern) drop_trial();
+    GB_TRY(rc);
+    pattern = trial;
+    (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = known.sched;
+    return GOOSEBERRY_SUCCESS;
   }
   const size_t xb = static_cast<size_t>(a.ncols) * (width == GB_CSR_VALUES_F32 ? 4 : 8);
   const size_t yb = static_cast<size_t>(a.nrows) * (width == GB_CSR_VALUES_F32 ? 4 : 8);
   void * x = nullptr;
   void * y = nullptr;
-  GB_TRY(dev_alloc(&x, std::max<size_t>(xb, 8)));
-  GB_TRY(dev_alloc(&y, std::max<size_t>(yb, 8)));
-  GB_CUDA_TRY(cudaMemsetAsync(x, 0, std::max<size_t>(xb, 8), stream));
+  int rc = dev_alloc(&x, std::max<size_t>(xb, 8));
+  if (rc == GOOSEBERRY_SUCCESS) rc = dev_alloc(&y, std::max<size_t>(yb, 8));
+  if (rc == GOOSEBERRY_SUCCESS &&
+      cudaMemsetAsync(x, 0, std::max<size_t>(xb, 8), stream) != cudaSuccess) {
+    set_error("autotune: %s", cudaGetErrorString(cudaGetLastError()));
+    rc = GOOSEBERRY_ERROR_UNKNOWN;
+  }
+  if (rc != GOOSEBERRY_SUCCESS) {
+    dev_free(x);
+    dev_free(y);
+    drop_trial();
+    return rc;
+  }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -770,20 +798,8 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
     bool pattern = false;
   };
   std::vector<Cand> cands;
-  const bool short_rows = a.plan.p99 <= 64 && a.plan.max_row <= 4096;
   if (short_rows) cands.push_back({1024, GB_SCHED_ROW});
-  SpmvPattern * trial = nullptr;
-  if (short_rows) {
-    const int prc = build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &trial, stream);
-    if (prc != GOOSEBERRY_SUCCESS) {
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      dev_free(x);
-      dev_free(y);
-      return prc;
-    }
-    if (trial) cands.push_back({1024, GB_SCHED_ROW, true});
-  }
+  if (trial) cands.push_back({1024, GB_SCHED_ROW, true});
   for (uint32_t t : {128u, 256u, 512u}) cands.push_back({t, GB_SCHED_WTILE});
   cands.push_back({static_cast<uint32_t>(32 * kWmKt), GB_SCHED_WMERGE});
   const void * vals = width == GB_CSR_VALUES_F32 ? static_cast<const void *>(a.val32)
@@ -798,7 +814,6 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   }
   float best = 1e30f;
   TuneChoice choice{default_schedule(a.plan), a.plan.tile_items};
-  int rc = GOOSEBERRY_SUCCESS;
   for (const Cand & cd : cands) {
     pattern = cd.pattern ? trial : nullptr;
     rc = rebuild_plan(a, cd.tile, stream);
@@ -840,10 +855,7 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   dev_free(x);
   dev_free(y);
   pattern = rc == GOOSEBERRY_SUCCESS && choice.pattern ? trial : nullptr;
-  if (trial && !pattern) {
-    cudaStreamSynchronize(stream);
-    free_spmv_pattern(trial);
-  }
+  if (!pattern) drop_trial();
   GB_TRY(rc);
   GB_TRY(rebuild_plan(a, choice.tile_items, stream));
   (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = choice.sched;
@@ -1046,6 +1058,30 @@ int gb_csr_get_info(const gb_csr_t * a, gb_csr_info_t * info) {
   info->schedule = a->sched64;
   info->schedule_f32 = a->sched32;
   info->tile_items = a->plan.tile_items;
+  return GOOSEBERRY_SUCCESS;
+}
+
+int gb_csr_row_form(const gb_csr_t * a, unsigned value_width, int * form) {
+  GB_CHECK_INPUT(a && form, "NULL argument");
+  const bool f32 = value_width == GB_CSR_VALUES_F32;
+  *form = (f32 ? a->sched32 : a->sched64) == GB_SCHED_ROW
+              ? gb::pattern_form(f32 ? a->pat32 : a->pat64)
+              : GB_ROWS_PLAIN;
+  return GOOSEBERRY_SUCCESS;
+}
+
+int gb_csr_compress_rows(gb_csr_t * a, unsigned value_width) {
+  GB_CHECK_INPUT(a != nullptr, "matrix is NULL");
+  const bool f32 = value_width == GB_CSR_VALUES_F32;
+  GB_CHECK_INPUT(f32 ? a->val32 != nullptr : a->val64 != nullptr,
+      "the matrix holds no values of this width");
+  gb::SpmvPattern * p = nullptr;
+  GB_TRY(gb::build_spmv_pattern(*a, f32, &p, nullptr));
+  GB_CHECK_INPUT(p != nullptr, "the rows do not repeat (at most 7 entries, 256 distinct rows or "
+      "lists of column offsets)");
+  gb::drop_pattern(*a, value_width);
+  (f32 ? a->pat32 : a->pat64) = p;
+  (f32 ? a->sched32 : a->sched64) = GB_SCHED_ROW;
   return GOOSEBERRY_SUCCESS;
 }
 

@@ -139,8 +139,21 @@ GOOSEBERRY_API int gb_csr_set_schedule(gb_csr_t * a, unsigned value_width, int s
  * of column offsets, also the row schedule over a compressed copy with its
  * results, reported as GB_SCHED_ROW; gb_csr_set_schedule drops it); the
  * choice is cached per process under a key of (row-length quantiles, nrows,
- * nnz, value width) so equal-shaped matrices skip the timing.  Synchronous. */
+ * nnz, value width, form of the compressed copy) so equal-shaped matrices skip
+ * the timing.  Synchronous. */
 GOOSEBERRY_API int gb_csr_autotune(gb_csr_t * a, unsigned value_width, gb_stream_t stream);
+
+/* What the row schedule reads: the CSR arrays, a byte a row for its column
+ * offsets (values from the CSR array), or a byte a row for all of it. */
+typedef enum gb_row_form {
+  GB_ROWS_PLAIN = 0,
+  GB_ROWS_PATTERNS = 1,
+  GB_ROWS_CLASSES = 2
+} gb_row_form_t;
+GOOSEBERRY_API int gb_csr_row_form(const gb_csr_t * a, unsigned value_width, int * form);
+/* Take the row schedule over the compressed copy without timing it.
+ * INVALIDINPUT, and no change, for a matrix that has none. */
+GOOSEBERRY_API int gb_csr_compress_rows(gb_csr_t * a, unsigned value_width);
 
 /* Run the SpMV tile planner on a HOST rowptr (no GPU involved).  Writes the
  * tile and long-row counts; when tiles != NULL (room for max_tiles) also the
