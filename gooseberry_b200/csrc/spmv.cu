@@ -746,7 +746,10 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   drop_pattern(a, width);
   const bool short_rows = a.plan.p99 <= 64 && a.plan.max_row <= 4096;
   SpmvPattern * trial = nullptr;
-  if (short_rows) GB_TRY(build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &trial, stream));
+  // (a compressed copy that there is no memory for is one candidate less)
+  if (short_rows &&
+      build_spmv_pattern(a, width == GB_CSR_VALUES_F32, &trial, stream) != GOOSEBERRY_SUCCESS)
+    cudaGetLastError();
   const auto drop_trial = [&] {
     if (!trial) return;
     cudaStreamSynchronize(stream);
@@ -774,8 +777,21 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   const size_t yb = static_cast<size_t>(a.nrows) * (width == GB_CSR_VALUES_F32 ? 4 : 8);
   void * x = nullptr;
   void * y = nullptr;
-  int rc = dev_alloc(&x, std::max<size_t>(xb, 8));
-  if (rc == GOOSEBERRY_SUCCESS) rc = dev_alloc(&y, std::max<size_t>(yb, 8));
+  const auto vectors = [&]() -> int {
+    GB_TRY(dev_alloc(&x, std::max<size_t>(xb, 8)));
+    const int r = dev_alloc(&y, std::max<size_t>(yb, 8));
+    if (r == GOOSEBERRY_SUCCESS) return r;
+    dev_free(x);
+    x = nullptr;
+    return r;
+  };
+  int rc = vectors();
+  const bool all = rc == GOOSEBERRY_SUCCESS || !trial;  // else: timed without the compressed copy
+  if (!all) {
+    cudaGetLastError();
+    drop_trial();
+    rc = vectors();
+  }
   if (rc == GOOSEBERRY_SUCCESS &&
       cudaMemsetAsync(x, 0, std::max<size_t>(xb, 8), stream) != cudaSuccess) {
     set_error("autotune: %s", cudaGetErrorString(cudaGetLastError()));
@@ -859,6 +875,7 @@ int autotune(gb_csr & a, unsigned width, cudaStream_t stream) {
   GB_TRY(rc);
   GB_TRY(rebuild_plan(a, choice.tile_items, stream));
   (width == GB_CSR_VALUES_F32 ? a.sched32 : a.sched64) = choice.sched;
+  if (!all) return GOOSEBERRY_SUCCESS;  // not a choice among all candidates: not kept
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_tune_cache[key] = choice;
   return GOOSEBERRY_SUCCESS;
