@@ -56,6 +56,7 @@ SCHED_NAMES = {0: "auto", 1: "thread", 2: "group4", 3: "group8", 4: "warp", 5: "
 CG_F64, CG_MIXED = 0, 1
 CG_PERSISTENT = 0x100
 CG_PLAIN_ENTRIES = 0x200
+CG_NO_CHIP = 0x400
 ROWS_PLAIN, ROWS_PATTERNS, ROWS_CLASSES = 0, 1, 2
 CHIP_FAULT_NONE, CHIP_FAULT_MISSING, CHIP_FAULT_LATE, CHIP_FAULT_SHORT = 0, 1, 2, 3
 CHIP_FAULT_REFUSED = 4
@@ -670,11 +671,11 @@ class CgSolver:
     """CG workspace bound to one matrix (``gb_cg_t``)."""
 
     def __init__(self, A: CsrMatrix, mode: int = CG_F64, persistent: bool = False,
-                 plain_entries: bool = False):
+                 plain_entries: bool = False, on_chip: bool = True):
         self.A = A
         h = C.c_void_p()
         flags = mode | (CG_PERSISTENT if persistent else 0) | (
-            CG_PLAIN_ENTRIES if plain_entries else 0)
+            CG_PLAIN_ENTRIES if plain_entries else 0) | (0 if on_chip else CG_NO_CHIP)
         _check(lib().gb_cg_create(A._h, flags, C.addressof(h)), "gb_cg_create")
         self._h = h
 
@@ -797,8 +798,10 @@ class Server:
     systems, call ``step()`` repeatedly, collect results with ``poll()``."""
 
     def __init__(self, pool_bytes: int = 16 << 30, max_slots: int = 128,
-                 mode: int = CG_MIXED, iters_per_step: int = 16, tile_rows: int = 0):
-        cfg = _ServerConfig(pool_bytes, max_slots, mode, iters_per_step, tile_rows)
+                 mode: int = CG_MIXED, iters_per_step: int = 16, tile_rows: int = 0,
+                 on_chip: bool = True):
+        cfg = _ServerConfig(pool_bytes, max_slots, mode | (0 if on_chip else CG_NO_CHIP),
+                            iters_per_step, tile_rows)
         h = C.c_void_p()
         _check(lib().gb_server_create(C.addressof(cfg), C.addressof(h)), "gb_server_create")
         self._h = h

@@ -1408,7 +1408,8 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
       a->ncols);
   const bool want_persistent = (mode & GB_CG_PERSISTENT) != 0;
   const bool plain_entries = (mode & GB_CG_PLAIN_ENTRIES) != 0;
-  mode &= ~(GB_CG_PERSISTENT | GB_CG_PLAIN_ENTRIES);
+  const bool chip = (mode & GB_CG_NO_CHIP) == 0;
+  mode &= ~(GB_CG_PERSISTENT | GB_CG_PLAIN_ENTRIES | GB_CG_NO_CHIP);
   GB_CHECK_INPUT(mode == GB_CG_F64 || mode == GB_CG_MIXED, "unknown CG mode %d", mode);
   GB_TRY(pinned_slot_alloc(sizeof(int), reinterpret_cast<void **>(&s->cancel_h),
       reinterpret_cast<void **>(&s->cancel_d)));
@@ -1417,7 +1418,7 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
     s->mode = mode;
     s->n = a->nrows;
     GB_TRY(mixed_create(a, plain_entries, &s->mixed));
-    if (!try_mixed_on_chip(a, plain_entries, s)) {
+    if (!chip || !try_mixed_on_chip(a, plain_entries, s)) {
       GB_TRY(mixed_past_chip(s->mixed));
       GB_TRY(mixed_ensure_graphs(s->mixed));
     }
@@ -1482,7 +1483,7 @@ int create_cg(const gb_csr * a, int mode, gb_cg * s) {
   GB_TRY(pinned_slot_alloc(2 * sizeof(CgStatus), reinterpret_cast<void **>(&s->host_status),
       nullptr));
   if (want_persistent) GB_TRY(setup_persistent(a, s));
-  else if (s->sched == GB_SCHED_ROW && setup_resident(a, plain_entries, s) != GOOSEBERRY_SUCCESS) {
+  else if (chip && s->sched == GB_SCHED_ROW && setup_resident(a, plain_entries, s) != GOOSEBERRY_SUCCESS) {
     cudaGetLastError();  // no memory for the solve on the chip
     drop_resident(s);
   }

@@ -752,6 +752,7 @@ struct gb_server {
   bool inflight = false;
   gb_server_stats_t stats{};
   // solves on the chip
+  bool chip = true;
   int device = 0;
   unsigned char * d_ctl = nullptr;      // [max_slots] control blocks
   unsigned char * h_pin = nullptr;      // [max_slots] pinned blocks
@@ -852,7 +853,9 @@ void destroy_server(gb_server * s) {
   delete s;
 }
 
-int create_server(const gb_server_config_t & cfg, gb_server * s) {
+int create_server(gb_server_config_t cfg, gb_server * s) {
+  s->chip = (cfg.mode & GB_CG_NO_CHIP) == 0;
+  cfg.mode &= ~GB_CG_NO_CHIP;
   GB_CHECK_INPUT(cfg.pool_bytes >= (1u << 20), "pool_bytes must be at least 1 MiB");
   GB_CHECK_INPUT(cfg.max_slots >= 1 && cfg.max_slots <= 4096, "max_slots must be in [1, 4096]");
   GB_CHECK_INPUT(cfg.mode == GB_CG_MIXED || cfg.mode == GB_CG_F64, "mode must be GB_CG_MIXED or GB_CG_F64");
@@ -1041,7 +1044,7 @@ int submit(gb_server & s, uint64_t id, dim_t n, const ind_t * rowptr, const dim_
     GB_CHECK_INPUT(ntiles <= kMaxTiles, "request needs %zu tiles, more than %zu", ntiles,
         kMaxTiles);
     for (uint32_t r = 0; r < n; r += T) q.tiles.push_back(SrvTile{0, r, std::min(T, n - r), 0});
-    return plan_on_chip(s, q, maxrow);
+    return s.chip ? plan_on_chip(s, q, maxrow) : GOOSEBERRY_SUCCESS;
   }();
   if (rc != GOOSEBERRY_SUCCESS) {
     if (q.stage_len) s.stage_alloc.release(q.stage_off, q.stage_len);

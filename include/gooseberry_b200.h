@@ -301,6 +301,12 @@ typedef enum gb_cg_mode {
  * instead. */
 #define GB_CG_PLAIN_ENTRIES 0x200
 
+/* OR-ed into the mode of gb_cg_create or gb_server_config_t: no solves on the
+ * chip.  The graph-replayed kernels, or the batch, then share the SMs with
+ * other streams kernel by kernel, where a launch on the chip holds them for
+ * about 10 ms. */
+#define GB_CG_NO_CHIP 0x400
+
 typedef enum gb_cg_status {
   GB_CG_CONVERGED = 0,  /* ||r|| <= tolerance                                 */
   GB_CG_MAXITER = 1,    /* iteration limit reached first                      */
@@ -439,7 +445,7 @@ typedef struct gb_server gb_server_t;
 typedef struct gb_server_config {
   size_t pool_bytes;        /* device memory for resident solves             */
   uint32_t max_slots;       /* resident solves at most                       */
-  int mode;                 /* GB_CG_MIXED or GB_CG_F64                      */
+  int mode;                 /* GB_CG_MIXED or GB_CG_F64, | GB_CG_NO_CHIP     */
   uint32_t iters_per_step;  /* CG iterations of the batch per gb_server_step
                                (>= 1)                                        */
   uint32_t tile_rows;       /* rows per work tile (a power of two in
