@@ -938,9 +938,13 @@ int tile_rows_for(gb_server & s, const Request & q, uint32_t maxrow, uint32_t * 
 // shape of that solve.  The rows are checked already.
 int plan_on_chip(gb_server & s, Request & q, uint32_t maxrow) {
   q.npat = 0;
-  if (maxrow < 1 || maxrow > 7) return GOOSEBERRY_SUCCESS;
-  uint32_t half = 0;
-  uint32_t last = 0;
+  if (maxrow < 1 || maxrow > 7 ||
+      q.n > static_cast<uint64_t>(srv_rows_per_cta(q.n)) * chip_capacity(s))
+    return GOOSEBERRY_SUCCESS;
+  uint32_t half = 0, last = 0;
+  // the lists by a hash of theirs, linear probing
+  constexpr uint32_t kSlots = 4 * kSrvPatMax;
+  uint16_t slot[kSlots] = {};  // list + 1
   for (uint32_t r = 0; r < q.n; ++r) {
     const uint32_t b = q.rowptr[r], l = q.rowptr[r + 1] - b;
     const auto is = [&](uint32_t p) {
@@ -950,22 +954,30 @@ int plan_on_chip(gb_server & s, Request & q, uint32_t maxrow) {
         if (q.rowind[b + j] - r != static_cast<uint32_t>(o[j])) return false;
       return true;
     };
-    uint32_t p = last;  // mostly the row before has it
-    if (p >= q.npat || !is(p)) {
-      for (p = 0; p < q.npat && !is(p); ++p) {
-      }
-      if (p == q.npat) {
-        if (q.npat == kSrvPatMax) return GOOSEBERRY_SUCCESS;
-        int32_t * o = q.pats + q.npat++ * kPatMax;
-        for (uint32_t j = 0; j + 1 < static_cast<uint32_t>(kPatMax); ++j) {
-          o[j] = j < l ? static_cast<int32_t>(q.rowind[b + j] - r) : 0;
-          half = std::max(half, static_cast<uint32_t>(std::abs(static_cast<int64_t>(o[j]))));
+    if (last >= q.npat || !is(last)) {  // mostly the row before has the same
+      uint32_t h = l;
+      for (uint32_t j = 0; j < l; ++j) h = (h ^ (q.rowind[b + j] - r)) * 0x9e3779b1u;
+      for (h >>= 16;; ++h) {
+        uint16_t & at = slot[h % kSlots];
+        if (at == 0) {
+          if (q.npat == kSrvPatMax) return GOOSEBERRY_SUCCESS;
+          last = q.npat++;
+          at = static_cast<uint16_t>(q.npat);
+          int32_t * o = q.pats + last * kPatMax;
+          for (uint32_t j = 0; j + 1 < static_cast<uint32_t>(kPatMax); ++j) {
+            o[j] = j < l ? static_cast<int32_t>(q.rowind[b + j] - r) : 0;
+            half = std::max(half, static_cast<uint32_t>(std::abs(static_cast<int64_t>(o[j]))));
+          }
+          o[kPatMax - 1] = static_cast<int32_t>(l);
+          break;
         }
-        o[kPatMax - 1] = static_cast<int32_t>(l);
+        if (is(at - 1u)) {
+          last = at - 1u;
+          break;
+        }
       }
     }
-    last = p;
-    q.codes[r] = static_cast<uint8_t>(p);
+    q.codes[r] = static_cast<uint8_t>(last);
   }
   // room beside the request's own arrays (admit lays them out)
   const size_t extra = align256(32ull * q.npat) + align256(q.n);
