@@ -748,6 +748,11 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
       else if (rnorm <= sh.tol) status = GB_CG_CONVERGED;
       else if (a.niter && it >= a.niter) status = GB_CG_MAXITER;
       else running = true;
+      if (!running && blockIdx.x == 0 && tid == 0) {
+        // here, not behind the loop: alive there, they cost 1-3% of every iteration
+        a.out->pap = pap;
+        a.out->beta = rr_new / rr;
+      }
     }
     if (a.hist && blockIdx.x == 0 && tid == T - 1 && it <= a.hist_len)
       a.hist[it - 1] = sqrt(rr_new);
@@ -769,8 +774,6 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     a.out->iter = it;
     a.out->rr = rr;
     a.out->bnorm = sh.bnorm;
-    a.out->pap = pap;
-    a.out->beta = beta;
     a.out->ran = it - (a.resume ? a.it0 : 0);
     a.out->t1 = res_ns();
     a.out->epoch = epoch;
