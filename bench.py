@@ -51,6 +51,19 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback 6.65 TB/s"
 
 
+def smem_peak():
+    """GB/s between shared memory and registers: 128 bytes a clock and SM."""
+    import torch
+    mhz = 1965.0
+    try:
+        with open(PEAKS_PATH) as f:
+            mhz = float(json.load(f)["sm_max_mhz"])
+    except Exception:
+        pass
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return 0.128 * sms * mhz, f"128 bytes a clock on {sms} SMs at {mhz:.0f} MHz"
+
+
 def cg_a_kernel_name(entry_bytes, row_bytes):
     """The FP64 CG's A kernel for the solver's matrix layout (stored bytes per
     entry and per row)."""
@@ -319,21 +332,24 @@ def run_cg_laplace(args, dist: Dist):
     h2d = 4 * (n + 1) + 4 * nnz + 8 * nnz + 8 * n
     d2h = 8 * n
 
-    # a solve on the chip is one launch: the matrix's codes and every vector
-    # stay in shared memory and registers, so HBM sees 9 + 16 bytes a row once
-    # and the iterations' bytes (as the two-kernel form moves them) never leave
-    # the SMs
+    # a solve on the chip keeps the matrix's codes and every vector in shared
+    # memory and registers (HBM sees 9 + 16 bytes a row once, and 48 a row for
+    # each further launch of about 10 ms), so what bounds it is the bytes that
+    # its iterations move between shared memory and registers: a row's p twice,
+    # its nnz/n entries' p, its own p, code and Ap, Ap again, x twice and p
     on_chip = results[-1].kernel_launches < iters
     peak, peak_src = hbm_peak()
     ach_a = bytes_a / (ms_a * 1e-3) / 1e9
     ach_a_stored = bytes_a_stored / (ms_a * 1e-3) / 1e9
     if on_chip:
         launch_ms = t_local / args.steps * 1e3
-        moved = (bytes_a + bytes_b) * iters
+        moved = (8.0 * nnz + (8 * 8 + 1) * n) * iters
+        peak, peak_src = smem_peak()
         roofline = {
-            "bound": "latency (two exchanges between the SMs and a shared-memory row loop "
-                     "an iteration)",
-            "kernel": "cg_resident_kernel (the whole solve; vectors and value codes on the SMs)",
+            "bound": "shared memory, and the latency of two exchanges between the SMs an "
+                     "iteration",
+            "kernel": "cg_resident_kernel (all launches of a solve; vectors and row codes on "
+                      "the SMs)",
             "achieved": moved / (launch_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
             "frac": moved / (launch_ms * 1e-3) / 1e9 / peak,
             "traffic": ncu_traffic("cg_resident_laplace1024"),
@@ -341,7 +357,7 @@ def run_cg_laplace(args, dist: Dist):
             "bytes_per_launch_stored": S.row_bytes() * (n + 1) + 16 * n,
             "on_chip": True, "l2_resident": False,
             "frac_textbook_per_step": (bytes_textbook * iters * args.steps / t_local / 1e9)
-                                      / peak,
+                                      / hbm_peak()[0],
         }
     else:
         roofline = {

@@ -45,7 +45,7 @@
 //                      or 8 values (doubles, or floats when exact) per row
 //
 // A pattern matrix whose vectors fit the SMs is solved by cg_resident.cu
-// instead, in one launch with the vectors on the chip.
+// instead, with the vectors on the chip.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>

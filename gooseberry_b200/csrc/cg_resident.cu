@@ -3,8 +3,8 @@
 // The graph-replayed solver (cg.cu) streams r, p, Ap and x through L2 twice
 // per iteration (about 90 bytes a row) and pays two dependent launches.  A
 // system whose vectors fit the SMs' shared memory and registers needs
-// neither: here ONE cooperative launch runs the whole solve, one CTA per SM,
-// each CTA owning a contiguous block of rows for its whole life.
+// neither: here cooperative launches of many iterations run the solve, one CTA
+// per SM, each CTA owning a contiguous block of rows for its whole life.
 //
 //   shared memory  p over the CTA's rows and H rows on either side (H = the
 //                  matrix's half bandwidth), Ap, x, the row patterns, and the
@@ -43,8 +43,8 @@
 // p.Ap of the next, and overwritten only after that all-reduce.
 //
 // Measured per iteration (us, B200), graph path -> here: 1024^2 Laplacian 20.9
-// -> 8.4; variable coefficients 1024^2 23.9 -> 11.7, 400^2 9.0 -> 4.1, 96^2 7.0
-// -> 3.3, 64^3 12.5 -> 7.8.  What an iteration of the 1024^2 Laplacian (7,086
+// -> 8.6; variable coefficients 1024^2 23.9 -> 11.7, 400^2 9.0 -> 4.1, 96^2 7.0
+// -> 3.3, 64^3 12.5 -> 8.1.  What an iteration of the 1024^2 Laplacian (7,086
 // rows a CTA) spends, in clocks of 16,500: row sums 5,200 (shared-memory
 // loads: 15 wavefronts a 32-row sum, floor 3,400), p updates 1,500, the
 // exchanges 2,600 and 5,900 (the second as long as the x update and the
@@ -300,10 +300,10 @@ __device__ __forceinline__ bool res_sum_fixed(const ResArgs & a, ResShared & sh,
 
 // Sum of every CTA's `local` (over its threads), the same bits in every CTA.
 // `prev`: a sum of about this size, the same in every CTA (0: unknown).  Warps
-// 1.. run `hidden` while warp 0 exchanges the sums, and warp 0
-// runs `sent` between its send and its wait.  Returns false when a wait was
-// given up, in every thread of the CTA alike: sh.bad is written between the two
-// barriers here, and elsewhere only behind a barrier that follows.
+// 1.. run `hidden` while warp 0 exchanges the sums, and warp 0 runs `sent` between
+// its send and its wait.  Returns false when a wait was given up, in every thread
+// of the CTA alike: sh.bad is written between the two barriers here, and elsewhere
+// only behind a barrier that follows.
 template <int T, class F, class S>
 __device__ __forceinline__ bool res_allreduce(const ResArgs & a, ResShared & sh, ResSums & st,
     uint32_t & epoch, double local, double prev, F && hidden, S && sent, double * total) {
@@ -602,7 +602,8 @@ __global__ void __launch_bounds__(T, 1) cg_resident_kernel(const ResArgs a) {
     sh.rr_far = tol > 1e-140 ? tol * tol * (1.0 + 1e-14) : INFINITY;
   }
   __syncthreads();
-  unsigned long long it = a.resume ? a.it0 : 0, t_a = 0, t_b = 0;  // t_a, t_b: ns in A and B (a.timed)
+  unsigned long long it = a.resume ? a.it0 : 0;
+  unsigned long long t_a = 0, t_b = 0;  // ns in A and B (a.timed)
   int status = GB_CG_MAXITER;
   bool running = ok;
   if (rr == 0.0) {

@@ -1,7 +1,7 @@
 // serve.cu -- batched CG serving: many uneven solves resident at once,
 // continuous batching, admission by device-memory footprint.  Requests whose
-// systems fit the SMs run there from start to end, side by side (see "solves
-// on the chip" below); the batch described next serves the others.
+// systems fit the SMs are solved there, side by side (see "solves on the chip"
+// below); the batch described next serves the others.
 //
 // Reference: one cgd call (src/cgd.c:40-129) runs at a time from the CLI
 // (src/gooseberry_bin.c:2078-2091).  Here every resident solve owns a slot:
@@ -93,10 +93,10 @@ constexpr size_t kMaxTiles = 1u << 20;
 //
 // A request whose matrix is a pattern matrix (rows of at most 7 entries, at
 // most 256 lists of column offsets) and whose rows fit the SMs' shared memory
-// is run from start to end by one launch of the on-chip solver
-// (cg_resident.cu) on as many SMs as it needs, beside those of other requests;
-// steps start queued solves as SMs come free and collect finished ones.  The
-// batch below serves the rest.
+// is solved by launches of the on-chip solver (cg_resident.cu), of about 10 ms
+// each, on as many SMs as it needs, beside those of other requests; steps start
+// them as SMs come free and collect the ended ones.  The batch below serves the
+// rest, beside them.
 //
 // The batch streams every vector of every solve through L2 or HBM each
 // iteration; on the chip only the edge values and two sums cross L2.  Measured
